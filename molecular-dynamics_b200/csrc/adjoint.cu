@@ -118,8 +118,8 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
             double4 xj[kHb], wj[kHb];
 #pragma unroll
             for (int b = 0; b < kHb; ++b) {
-                xj[b] = xs[ej[b]];
-                wj[b] = w[er[b]];
+                xj[b] = ldg_d4(xs + ej[b]);
+                wj[b] = ldg_d4(w + er[b]);
             }
 #pragma unroll
             for (int b = 0; b < kHb; ++b) {
@@ -225,7 +225,7 @@ k_adj_init(const double4* __restrict__ pos, const int* __restrict__ img, const i
         const int n = min(nbn[i], nbcap);
         for (int k = 0; k < n; ++k) {
             const int j = (int)(__ldg(nbl + nl_index(k, i, stride)) >> kCodeBits);
-            const double4 q = pos[j];
+            const double4 q = ldg_d4(pos + j);
             const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
             const double s = dx * dx + dy * dy + dz * dz;
             if (s < rc2) {

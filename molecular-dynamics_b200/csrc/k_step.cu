@@ -45,12 +45,6 @@ struct DemArgs {
     double rc2, dn, dt_, k, mu, radius;
 };
 
-__device__ __forceinline__ double4 ldg_d4(const double4* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    double2 a = __ldg(q), b = __ldg(q + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
-}
-
 // writes the per-block partial of quantity q (kThermoQ-major layout)
 __device__ __forceinline__ void put_partial(double* part, int q, double v, double* scratch) {
     double r = block_sum(v, scratch);

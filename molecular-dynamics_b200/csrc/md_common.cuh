@@ -32,6 +32,19 @@ __device__ __forceinline__ double len2_strict(double x, double y, double z) {
     return dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
 }
 
+// ---- 32-byte gathers -------------------------------------------------------
+// One 256-bit load (sm_100) of a slot's position or velocity, for data the kernel does not write.
+// The FP64 force kernels are bound by L1, which spends its time on the scattered addresses of a
+// gather and not on its bytes: with two 128-bit loads per neighbour the FP64 LJ kernel took 52.0 us
+// at 131,072 atoms and 166 us at 524,288, with one 256-bit load 43.8 and 140 us; the contact DEM
+// kernel 35.0 -> 31.7 us (FP64, 223,488 grains) and 28.2 -> 27.0 us (mixed).  The per-slot arrays
+// start on 256-byte boundaries, so every element is 32-byte aligned.
+__device__ __forceinline__ double4 ldg_d4(const double4* p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
 // ---- packed per-atom integer triplets (10 bits per axis, modulo 1024) -----
 __device__ __forceinline__ int pack3(int a, int b, int c) {
     return (a & 1023) | ((b & 1023) << 10) | ((c & 1023) << 20);
