@@ -215,7 +215,7 @@ int md_profile_get(int kernel_id, long long *launches, double *total_ms);
 void md_profile_reset(void);
 /* Number of kernel launches issued since md_initialize_grid. */
 long long md_kernel_launches(void);
-/* Device bytes held by the library. */
+/* Device bytes asked for by the current grid (blocks kept from earlier grids are not counted). */
 long long md_device_bytes(void);
 
 /* Runs `steps` timesteps of the md driver loop (main.cpp:715-776) natively:

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <mutex>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -56,14 +57,106 @@ void launched(int kernel_id) {
     if (e != cudaSuccess) set_error(MD_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
+// Device blocks a closed grid leaves are kept for the next one.  A grid takes some twenty of them,
+// and cudaMalloc / cudaFree cost more than a short run's steps: opening and closing a grid took 2.4
+// ms at 2,048 atoms and 3.5 ms at 131,072 on a quiet host (100 steps of the mixed form: 2.1 and 3.9
+// ms), and 20-50 ms where other processes of the host allocate at the same time.  Kept blocks are
+// bounded in number and bytes and go back to the device at md_mpi_finalize, or at once when an
+// allocation fails.  A block is handed out again only after a device synchronisation that follows
+// its release, as cudaFree waits for the work that uses a block.
+namespace {
+struct Block {
+    void* p;
+    size_t bytes;
+    int device;
+    bool idle;  // a device synchronisation followed its release
+};
+constexpr size_t kKeepBytes = (size_t)1 << 30;
+constexpr size_t kKeepBlocks = 64;
+std::mutex blocks_mutex;
+std::vector<Block> live_blocks, kept_blocks;
+
+void free_block(const Block& b) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    if (cur != b.device) cudaSetDevice(b.device);
+    if (cudaFree(b.p) != cudaSuccess) cudaGetLastError();
+    if (cur != b.device) cudaSetDevice(cur);
+}
+
+void free_kept_locked() {
+    for (const Block& b : kept_blocks) free_block(b);
+    kept_blocks.clear();
+}
+}  // namespace
+
+void release_kept_blocks() {
+    std::lock_guard<std::mutex> lock(blocks_mutex);
+    free_kept_locked();
+}
+
 void dev_alloc(void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
-    if (cuda_ok(cudaMalloc(p, bytes), "cudaMalloc")) g_state.dev_bytes += (long long)bytes;
+    int device = 0;
+    if (!cuda_ok(cudaGetDevice(&device), "cudaGetDevice")) return;
+    std::lock_guard<std::mutex> lock(blocks_mutex);
+    // the smallest kept block that holds the request without wasting more than half of itself
+    int best = -1;
+    for (int k = 0; k < (int)kept_blocks.size(); ++k) {
+        const Block& b = kept_blocks[k];
+        if (b.device == device && b.bytes >= bytes && b.bytes <= 2 * bytes + 4096 &&
+            (best < 0 || b.bytes < kept_blocks[best].bytes))
+            best = k;
+    }
+    if (best >= 0 && !kept_blocks[best].idle) {
+        if (cuda_ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize")) {
+            for (Block& b : kept_blocks)
+                if (b.device == device) b.idle = true;
+        } else {
+            best = -1;
+        }
+    }
+    if (best >= 0) {
+        live_blocks.push_back(kept_blocks[best]);
+        kept_blocks.erase(kept_blocks.begin() + best);
+        *p = live_blocks.back().p;
+    } else {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation && !kept_blocks.empty()) {
+            cudaGetLastError();
+            free_kept_locked();
+            e = cudaMalloc(p, bytes);
+        }
+        if (!cuda_ok(e, "cudaMalloc")) {
+            *p = nullptr;
+            return;
+        }
+        live_blocks.push_back(Block{*p, bytes, device, false});
+    }
+    g_state.dev_bytes += (long long)bytes;
 }
 
 void dev_free(void** p) {
-    if (*p) cudaFree(*p);
+    if (!*p) return;
+    std::lock_guard<std::mutex> lock(blocks_mutex);
+    for (size_t k = 0; k < live_blocks.size(); ++k) {
+        if (live_blocks[k].p != *p) continue;
+        Block b = live_blocks[k];
+        b.idle = false;
+        live_blocks.erase(live_blocks.begin() + k);
+        // room for it: the longest-kept blocks go back to the device first
+        size_t total = b.bytes;
+        for (const Block& q : kept_blocks) total += q.bytes;
+        while (!kept_blocks.empty() && (total > kKeepBytes || kept_blocks.size() >= kKeepBlocks)) {
+            total -= kept_blocks.front().bytes;
+            free_block(kept_blocks.front());
+            kept_blocks.erase(kept_blocks.begin());
+        }
+        if (total <= kKeepBytes) kept_blocks.push_back(b);
+        else free_block(b);
+        break;
+    }
     *p = nullptr;
 }
 
@@ -247,6 +340,21 @@ std::vector<SlabItem> slab_items(State& s) {
     return v;
 }
 
+// the events and the copy stream of a grid
+void free_sync_objects(State& s) {
+    for (cudaEvent_t* e : {&s.ev_counted, &s.ev_scanned, &s.ev_status}) {
+        if (*e) cudaEventDestroy(*e);
+        *e = nullptr;
+    }
+    for (cudaEvent_t& e : s.thermo_ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    if (s.copy_stream) cudaStreamDestroy(s.copy_stream);
+    s.copy_stream = nullptr;
+    s.sync_device = -1;
+}
+
 void free_all(State& s) {
     for (SlabItem& it : slab_items(s)) *it.p = nullptr;  // carved from the slab, freed with it
     dfree(&s.slab);
@@ -259,30 +367,11 @@ void free_all(State& s) {
     dfree(&s.bmask);
     dfree(&s.nbl);
     dfree(&s.red_part);
-    if (s.ev_counted) {
-        cudaEventDestroy(s.ev_counted);
-        s.ev_counted = nullptr;
-    }
-    if (s.ev_scanned) {
-        cudaEventDestroy(s.ev_scanned);
-        s.ev_scanned = nullptr;
-    }
-    if (s.ev_status) {
-        cudaEventSynchronize(s.ev_status);
-        cudaEventDestroy(s.ev_status);
-        s.ev_status = nullptr;
-    }
+    // the events and the copy stream stay for the next grid (made anew when the device changes)
+    if (s.ev_status) cudaEventSynchronize(s.ev_status);
     s.status_pending = false;
-    if (s.copy_stream) {
-        cudaStreamSynchronize(s.copy_stream);
-        cudaStreamDestroy(s.copy_stream);
-        s.copy_stream = nullptr;
-    }
-    for (int k = 0; k < kThermoSlots; ++k) {
-        if (s.thermo_ev[k]) cudaEventDestroy(s.thermo_ev[k]);
-        s.thermo_ev[k] = nullptr;
-        s.thermo_slot_ticket[k] = -1;
-    }
+    if (s.copy_stream) cudaStreamSynchronize(s.copy_stream);
+    for (int k = 0; k < kThermoSlots; ++k) s.thermo_slot_ticket[k] = -1;
     dfree(&s.thermo_dev);
     dfree(&s.status_dev);
     s.scan_part_cap = 0;
@@ -375,18 +464,21 @@ bool allocate_state(State& s, int N, int nb_cap) {
     dalloc(&s.bcount, (size_t)2 * 27 * nblk + 1);  // border types (26) or migration classes (27), scanned
     s.nb_cap = list_rows(nb_cap > 0 ? nb_cap : 100);
     dalloc(&s.nbl, list_entries(s));
-    if (!s.ev_counted) TMD_CUDA(cudaEventCreateWithFlags(&s.ev_counted, cudaEventDisableTiming));
-    if (!s.ev_scanned) TMD_CUDA(cudaEventCreateWithFlags(&s.ev_scanned, cudaEventDisableTiming));
-    if (!s.ev_status) TMD_CUDA(cudaEventCreateWithFlags(&s.ev_status, cudaEventDisableTiming));
-    if (!s.copy_stream) TMD_CUDA(cudaStreamCreateWithFlags(&s.copy_stream, cudaStreamNonBlocking));
+    if (s.sync_device != s.device) {
+        free_sync_objects(s);
+        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_counted, cudaEventDisableTiming));
+        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_scanned, cudaEventDisableTiming));
+        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_status, cudaEventDisableTiming));
+        TMD_CUDA(cudaStreamCreateWithFlags(&s.copy_stream, cudaStreamNonBlocking));
+        for (int k = 0; k < kThermoSlots; ++k)
+            TMD_CUDA(cudaEventCreateWithFlags(&s.thermo_ev[k], cudaEventDisableTiming));
+        s.sync_device = s.device;
+    }
     dalloc(&s.thermo_dev, 8);
     dalloc(&s.status_dev, 1);
     if (!s.status_host) TMD_CUDA(cudaMallocHost((void**)&s.status_host, sizeof(DevStatus)));
     if (!s.thermo_host) TMD_CUDA(cudaMallocHost((void**)&s.thermo_host, kThermoSlots * 4 * sizeof(double)));
-    for (int k = 0; k < kThermoSlots; ++k) {
-        if (!s.thermo_ev[k]) TMD_CUDA(cudaEventCreateWithFlags(&s.thermo_ev[k], cudaEventDisableTiming));
-        s.thermo_slot_ticket[k] = -1;
-    }
+    for (int k = 0; k < kThermoSlots; ++k) s.thermo_slot_ticket[k] = -1;
     s.thermo_tickets = 0;
     TMD_CUDA(cudaMemsetAsync(s.status_dev, 0, sizeof(DevStatus), s.stream));
     TMD_CUDA(cudaMemsetAsync(s.thermo_dev, 0, 8 * sizeof(double), s.stream));
@@ -1173,6 +1265,8 @@ void md_mpi_initialize(void) {
 }
 void md_mpi_finalize(void) {
     if (g_state.alive) md_deallocate_grid();
+    free_sync_objects(g_state);
+    release_kept_blocks();
     comm().finalize();
 }
 void md_barrier(void) {  // this rank's device work done, then every rank's

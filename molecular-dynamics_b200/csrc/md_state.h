@@ -234,6 +234,7 @@ struct State {
     cudaEvent_t ev_counted = nullptr;  // the ghost count's readback (run_borders)
     cudaEvent_t ev_scanned = nullptr;  // the ghost offsets scanned (the readback waits on it)
     cudaStream_t copy_stream = nullptr;  // the ghost count's readback, beside the emit kernel
+    int sync_device = -1;              // device whose events and copy stream the grid holds (kept between grids)
     int scan_attr_device = -1;         // device whose k_scan_single shared-memory attribute is set
     unsigned long long* lb_tiles = nullptr;  // look-back scan: one word per tile (k_neigh.cu)
     int lb_tile_cap = 0;
@@ -362,7 +363,8 @@ void ensure_red_scratch(State& s, int n);
 
 // device memory helpers
 void dev_alloc(void** p, size_t bytes);
-void dev_free(void** p);
+void dev_free(void** p);       // kept for a later dev_alloc, within bounds
+void release_kept_blocks();    // the kept blocks back to the device
 template <class T>
 inline void dalloc(T** p, size_t n) { dev_alloc(reinterpret_cast<void**>(p), n * sizeof(T)); }
 template <class T>
