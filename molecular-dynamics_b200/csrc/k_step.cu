@@ -45,6 +45,7 @@ struct DemArgs {
     double rc2, dn, dt_, k, mu, radius;
 };
 
+
 // writes the per-block partial of quantity q (kThermoQ-major layout)
 __device__ __forceinline__ void put_partial(double* part, int q, double v, double* scratch) {
     double r = block_sum(v, scratch);
@@ -614,6 +615,254 @@ k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos,
     }
 }
 
+// ---- several lanes per atom (full lists, small systems) -------------------------
+// A thread per atom leaves the chip idle below ~64k atoms: at 2,048 atoms the mixed kernel ran 64
+// warps, each walking ~19 list quads one after the other, and took 18.9 us, as long as at 16,384
+// (19.6 us); the FP64 kernel 23.4 and 25.2 us.  Here L adjacent lanes share an atom: lane `sub`
+// takes the quads sub, sub + L, ..., so the chain of dependent gathers is L times shorter.  All
+// lanes of an atom end with its force, integrate it alike and share the writing of its images.
+// Chain ghosts have blocks of their own behind the atoms' blocks.
+
+// the images of atom i from its new position x, plane k by lane k % L
+template <int L, bool MIXED>
+__device__ __forceinline__ void push_images_lanes(int i, int sub, const double4& x, int N, const PushArgs& pa,
+                                                  double4* __restrict__ pos_n, float4* __restrict__ pos32_n,
+                                                  const double* alo, double rb_h) {
+    for (int k = sub; k < pa.planes; k += L) {
+        const int t = pa.slot[(size_t)k * pa.plane + i];
+        if (t < 0) return;
+        write_ghost<MIXED>(t, x, pa.gcode[t - N], pa, pos_n, pos32_n, alo, rb_h);
+    }
+}
+
+// chain ghosts of the blocks behind the atoms' blocks
+template <bool MIXED>
+__device__ __forceinline__ void push_chain_block(int block, const double4* __restrict__ pos, int N, const PushArgs& pa,
+                                                 double4* __restrict__ pos_n, float4* __restrict__ pos32_n,
+                                                 const double* alo, double rb_h) {
+    const int q = block * (int)blockDim.x + (int)threadIdx.x;
+    if (q < (pa.nchain_dev ? *pa.nchain_dev : pa.nchain))
+        push_chain<MIXED>(q, pos, N, pa, pos_n, pos32_n, alo, rb_h);
+}
+
+// The pair arithmetic and the FP64-path queue of k_lj_mixed_bf; the lanes' sums are added in FP64.
+template <int L, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
+__global__ void __launch_bounds__(kThreads)
+k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ pos, float4* __restrict__ frc32,
+                 double4* __restrict__ vel, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
+                 double* __restrict__ part, LjArgs a, int atom_blocks, double4* __restrict__ pos_n = nullptr,
+                 float4* __restrict__ pos32_n = nullptr, const int* __restrict__ rbk = nullptr,
+                 PushArgs pa = PushArgs()) {
+    __shared__ double scratch[kThreads / 32];
+    __shared__ int s_q[kQQ + 1][kThreads];
+    if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
+    double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
+    if ((int)blockIdx.x < atom_blocks) {
+        const int t = blockIdx.x * kThreads + threadIdx.x;
+        const int i = t / L, sub = t % L;
+        const bool act = i < a.N;
+        const int n = act ? min(nbn[i], a.nbcap) : 0;
+        const float4 ri = act ? pos32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float fx = 0.f, fy = 0.f, fz = 0.f, ef = 0.f, wf = 0.f;
+        double cx = 0.0, cy = 0.0, cz = 0.0;
+        int ncnt = 0, nq = 0;
+        const int nquad = (n + 3) >> 2;
+        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        for (int b = sub; b < nquad; b += L) {
+            const uint32_t cur[kB32] = {eq.x, eq.y, eq.z, eq.w};
+            float4 rj[kB32];
+#pragma unroll
+            for (int u = 0; u < kB32; ++u) rj[u] = __ldg(pos32 + (cur[u] >> kCodeBits));
+            if (b + L < nquad) eq = list_quad(nbl, b + L, i, a.stride);
+            unsigned slow = 0;
+#pragma unroll
+            for (int u = 0; u < kB32; ++u)
+                slow |= mixed_pair<THERMO>(cur[u], ri, rj[u], a, fx, fy, fz, ef, wf, ncnt) ? (1u << u) : 0u;
+            s_q[min(nq, kQQ)][threadIdx.x] = (b << kB32) | (int)slow;
+            nq += slow != 0u ? 1 : 0;
+        }
+        if (nq > kQQ) {  // more than the queue holds: this lane's quads again, FP64 pairs in place
+            fx = fy = fz = ef = wf = 0.f;
+            ncnt = 0;
+            const double4 pi = ldg_d4(pos + i);
+            for (int b = sub; b < nquad; b += L) {
+                const uint4 e4 = list_quad(nbl, b, i, a.stride);
+                const uint32_t c4[kB32] = {e4.x, e4.y, e4.z, e4.w};
+                for (int u = 0; u < kB32; ++u) {
+                    const int j = (int)(c4[u] >> kCodeBits);
+                    if (mixed_pair<THERMO>(c4[u], ri, __ldg(pos32 + j), a, fx, fy, fz, ef, wf, ncnt))
+                        fp64_lj<THERMO>(pi, j, pos, a, cx, cy, cz, e, w, ncnt);
+                }
+            }
+        } else if (nq > 0) {
+            const double4 pi = ldg_d4(pos + i);
+            for (int q = 0; q < nq; ++q) {
+                const int wq = s_q[q][threadIdx.x];
+                const uint4 e4 = list_quad(nbl, wq >> kB32, i, a.stride);
+                unsigned bits = (unsigned)wq & ((1u << kB32) - 1u);
+                while (bits) {
+                    const int u = __ffs(bits) - 1;
+                    bits &= bits - 1u;
+                    const uint32_t en = u == 0 ? e4.x : (u == 1 ? e4.y : (u == 2 ? e4.z : e4.w));
+                    fp64_lj<THERMO>(pi, (int)(en >> kCodeBits), pos, a, cx, cy, cz, e, w, ncnt);
+                }
+            }
+        }
+        double Fx = (double)fx + cx, Fy = (double)fy + cy, Fz = (double)fz + cz;
+        __syncwarp();
+#pragma unroll
+        for (int o = 1; o < L; o <<= 1) {
+            Fx += __shfl_xor_sync(0xffffffffu, Fx, o);
+            Fy += __shfl_xor_sync(0xffffffffu, Fy, o);
+            Fz += __shfl_xor_sync(0xffffffffu, Fz, o);
+        }
+        const float4 F = make_float4((float)Fx, (float)Fy, (float)Fz, 0.f);
+        if (act && sub == 0) frc32[i] = F;
+        if (FUSE) {
+            double4 v = act ? vel[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+            v.x += (double)F.x * a.h;
+            v.y += (double)F.y * a.h;
+            v.z += (double)F.z * a.h;
+            if (THERMO && sub == 0) ke = v.x * v.x + v.y * v.y + v.z * v.z;
+            if (INIT && act) {
+                double4 x = integrate_one(ldg_d4(pos + i), v, (double)F.x, (double)F.y, (double)F.z, a.dt_i, a.h_i);
+                x.w = 0.0;  // positions carry w = 0
+                if (sub == 0) {
+                    pos_n[i] = x;
+                    pos32_n[i] = rebased32(x, rbk[i], a.alo, a.rb_h);
+                }
+                if (PUSH) push_images_lanes<L, true>(i, sub, x, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
+            }
+            __syncwarp();  // every lane has read the velocity
+            if (act && sub == 0) vel[i] = v;
+        }
+        if (THERMO) {
+            e += (double)ef;
+            w += (double)wf;
+            cnt = (double)ncnt;
+        }
+    } else if (PUSH) {
+        push_chain_block<true>((int)blockIdx.x - atom_blocks, pos, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
+    }
+    if (THERMO) {
+        put_partial(part, 0, e, scratch);
+        put_partial(part, 1, w, scratch);
+        put_partial(part, 2, cnt, scratch);
+        if (FUSE) put_partial(part, 3, ke, scratch);
+    }
+}
+
+// FP64: bit-identical to k_lj_fp64, so an atom's pair forces are added one by one in list order.  A
+// round takes 4 L list entries (a quad per lane); the lanes put their pair forces into shared memory
+// and three lanes of the atom add one component each, in order, while the next round's quads load.
+// An entry outside the cutoff or past the list's end adds +0.0, which changes no bit of a sum that
+// starts at +0.0 (such a sum is never -0.0).
+template <int L, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
+__global__ void __launch_bounds__(kThreads)
+k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
+                const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, double* __restrict__ part, LjArgs a,
+                int atom_blocks, double4* __restrict__ pos_n = nullptr, PushArgs pa = PushArgs()) {
+    static_assert(L >= 4 && L <= 32, "three lanes of an atom add its force's components");
+    // pairs outside the cutoff evaluated too, without a branch: shorter chains (2,048 atoms, 8 lanes:
+    // step 12.9 -> 12.2 us) but more work (16,384 atoms, 4 lanes: 18.1 -> 19.2 us)
+    constexpr bool kFlat = L >= 8;
+    constexpr int kAtoms = 32 / L;       // atoms per warp
+    // a component's 4 L doubles of a round, and an atom's three components: strides that keep the
+    // 16-byte writes of eight lanes and the reads of an atom's three on different banks
+    constexpr int kRow = 4 * L + 2;
+    constexpr int kAtom = L == 4 ? 3 * kRow + 2 : 3 * kRow;
+    __shared__ double scratch[kThreads / 32];
+    __shared__ __align__(16) double s_p[kThreads / 32][kAtoms * kAtom];
+    if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
+    double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
+    if ((int)blockIdx.x < atom_blocks) {
+        const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int t = blockIdx.x * kThreads + threadIdx.x;
+        const int i = t / L, sub = t % L, at = lane / L;
+        const bool act = i < a.N;
+        const int n = act ? min(nbn[i], a.nbcap) : 0;
+        const double4 pi = act ? pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        double acc = 0.0;  // component `sub` of the force (sub < 3)
+        const int nquad = (n + 3) >> 2;
+        const int rounds = __reduce_max_sync(0xffffffffu, (nquad + L - 1) / L);
+        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        for (int r = 0; r < rounds; ++r) {
+            const int b = r * L + sub;
+            const uint32_t ent[kB64] = {eq.x, eq.y, eq.z, eq.w};
+            double4 pj[kB64];
+#pragma unroll
+            for (int u = 0; u < kB64; ++u) pj[u] = ldg_d4(pos + (ent[u] >> kCodeBits));
+            if (b + L < nquad) eq = list_quad(nbl, b + L, i, a.stride);
+            double p[3][kB64];
+#pragma unroll
+            for (int u = 0; u < kB64; ++u) {
+                const double dx = dsub(pi.x, pj[u].x), dy = dsub(pi.y, pj[u].y), dz = dsub(pi.z, pj[u].z);
+                const double rsq = len2_strict(dx, dy, dz);
+                const bool in = 4 * b + u < n && rsq < a.rc2;
+                double sr2 = 0.0, sr6 = 0.0, f = 0.0;
+                if (kFlat || in) {  // flat: every lane divides, the four divisions side by side
+                    sr2 = ddiv(1.0, !kFlat || in ? rsq : 1.0);
+                    sr6 = dmul(dmul(dmul(sr2, sr2), sr2), a.sigma6);
+                    f = dmul(dmul(dmul(dmul(48.0, sr6), dsub(sr6, 0.5)), sr2), a.eps);
+                }
+                p[0][u] = in ? dmul(dx, f) : 0.0;
+                p[1][u] = in ? dmul(dy, f) : 0.0;
+                p[2][u] = in ? dmul(dz, f) : 0.0;
+                if (THERMO && in) {
+                    e += 4.0 * a.eps * sr6 * (sr6 - 1.0);
+                    w += f * rsq;
+                    cnt += 1.0;
+                }
+            }
+            // entry 4 sub + 2 h + e of the round at h 2 L + 2 sub + e
+            double* row = s_p[wid] + at * kAtom;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    *reinterpret_cast<double2*>(row + c * kRow + h * 2 * L + 2 * sub) =
+                        make_double2(p[c][2 * h], p[c][2 * h + 1]);
+            __syncwarp();
+            if (sub < 3) {
+                const double* q = row + sub * kRow;
+#pragma unroll
+                for (int k = 0; k < 2 * L; ++k) {
+                    const double2 v = *reinterpret_cast<const double2*>(q + (k & 1) * 2 * L + (k >> 1) * 2);
+                    acc = dadd(dadd(acc, v.x), v.y);
+                }
+            }
+            __syncwarp();
+        }
+        const int base = lane & ~(L - 1);
+        const double fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
+                     fz = __shfl_sync(0xffffffffu, acc, base + 2);
+        if (act && sub == 0) frc[i] = make_double4(fx, fy, fz, 0.0);
+        if (FUSE) {  // core/compute.impala:108-116
+            double4 v = act ? vel[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+            v.x = dadd(v.x, dmul(fx, a.h));
+            v.y = dadd(v.y, dmul(fy, a.h));
+            v.z = dadd(v.z, dmul(fz, a.h));
+            if (THERMO && sub == 0) ke = v.x * v.x + v.y * v.y + v.z * v.z;
+            if (INIT && act) {  // positions carry w = 0
+                double4 x = integrate_one(pi, v, fx, fy, fz, a.dt_i, a.h_i);
+                x.w = 0.0;
+                if (sub == 0) pos_n[i] = x;
+                if (PUSH) push_images_lanes<L, false>(i, sub, x, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
+            }
+            __syncwarp();  // every lane has read the velocity
+            if (act && sub == 0) vel[i] = v;
+        }
+    } else if (PUSH) {
+        push_chain_block<false>((int)blockIdx.x - atom_blocks, pos, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
+    }
+    if (THERMO) {
+        put_partial(part, 0, e, scratch);
+        put_partial(part, 1, w, scratch);
+        put_partial(part, 2, cnt, scratch);
+        if (FUSE) put_partial(part, 3, ke, scratch);
+    }
+}
+
 // ---- DEM ----------------------------------------------------------------------
 // core/runtime.impala:203-247.  With the reference condition the contact
 // branch can never run (penetration r - 2R > 0 inside r < 2R); `fixed`
@@ -1024,11 +1273,58 @@ StepArgs step_args(const State& s, double dt) {
     return a;
 }
 
+// Lanes per atom of a full-list LJ force kernel (1: the thread-per-atom kernels).  More lanes
+// shorten the chain of gathers that bounds a small system; a system that fills the chip pays for
+// them (the sums across lanes, the FP64 form's exchange through shared memory).  Step times in us
+// (LJ liquid, rebuild every 20 steps included), 1 / 2 / 4 / 8 / 16 lanes:
+//   mixed  2,048 atoms 21 / 15.7 / 13.0 / 11.6 / 11.0    16,384  22 / 17.7 / 15.7 / 15.8 / 19.7
+//         42,592       25 / 21.6 / 20.4 / 26.5 / 31      70,304  28.6 / 26.4 / 30.1   87,808 33.3 / 33.6 / 35.8
+//   FP64   2,048 atoms 25.3 / - / 14.9 / 11.9 / 11.8      5,148  26.8 / - / 15.0 / 13.1 / 15.0
+//          7,488       25.6 / - / 15.0 / 15.0 / 17.0     32,000  28.2 / - / 24.3 / 32.5   42,592 29.1 / - / 35.8
+int force_lanes(int N, bool mixed) {
+    if (N <= 2048) return 16;
+    if (mixed) return N <= 16384 ? 8 : N <= 49152 ? 4 : N <= 81920 ? 2 : 1;
+    return N <= 7168 ? 8 : N <= 38912 ? 4 : 1;
+}
+
+// blocks of a full-list LJ force launch over N atoms and nchain chain ghosts
+int force_blocks(int N, int lanes, int nchain) {
+    if (lanes == 1) return nblocks(N + nchain, kThreads);
+    return nblocks((long long)N * lanes, kThreads) + nblocks(nchain, kThreads);
+}
+
+template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
+void launch_lj_mixed_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
+    k_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
+        s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a,
+        nblocks((long long)a.N * L, kThreads), INIT ? s.pos.b[1 - s.pc] : nullptr,
+        INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
+}
+
+template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
+void launch_lj_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
+    if (s.precision == 1) return launch_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
+    k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
+        s.pos.b[s.pc], s.frc.b[s.ac], s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a,
+        nblocks((long long)a.N * L, kThreads), INIT ? s.pos.b[1 - s.pc] : nullptr, pa);
+}
+
 // INIT: the kernels write the integrated locals into the other position buffer
 template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
-void launch_lj(State& s, const LjArgs& a, int nb, const PushArgs& pa = PushArgs()) {
+void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs& pa = PushArgs()) {
     double4* vel = s.vel.b[s.vc];
     double4* pn = INIT ? s.pos.b[1 - s.pc] : nullptr;
+    if constexpr (!HALF) {
+        switch (lanes) {
+            case 2:  // the mixed form only
+                if (s.precision == 1) return launch_lj_mixed_lanes<2, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
+                break;
+            case 4: return launch_lj_lanes<4, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
+            case 8: return launch_lj_lanes<8, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
+            case 16: return launch_lj_lanes<16, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
+            default: break;
+        }
+    }
     if (s.precision == 1) {
         if constexpr (HALF)
             k_lj_mixed_half<THERMO><<<nb, kThreads, 0, s.stream>>>(s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.nbn,
@@ -1093,8 +1389,9 @@ void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt) {
     a.hx = (float)(-s.geo.rb_h);
     a.hy = (float)(-s.geo.rb_h / 4.0);
     a.hz = (float)(-s.geo.rb_h / 16.0);
-    const int nb = nblocks(N, kThreads);
     const bool half = p.half;
+    const int lanes = half ? 1 : force_lanes(N, s.precision == 1);
+    const int nb = force_blocks(N, lanes, 0);
     const bool thermo = s.thermo != 0;
     if (thermo) ensure_red_scratch(s, kThermoQ * nb);
     if (half) {
@@ -1110,11 +1407,11 @@ void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt) {
         if (thermo) launch_lj<true, false, true>(s, a, nb);
         else launch_lj<true, false, false>(s, a, nb);
     } else if (fuse_final) {
-        if (thermo) launch_lj<false, true, true>(s, a, nb);
-        else launch_lj<false, true, false>(s, a, nb);
+        if (thermo) launch_lj<false, true, true>(s, a, nb, lanes);
+        else launch_lj<false, true, false>(s, a, nb, lanes);
     } else {
-        if (thermo) launch_lj<false, false, true>(s, a, nb);
-        else launch_lj<false, false, false>(s, a, nb);
+        if (thermo) launch_lj<false, false, true>(s, a, nb, lanes);
+        else launch_lj<false, false, false>(s, a, nb, lanes);
     }
     launched(K_FORCE_LJ);
     prof_end(K_FORCE_LJ);
@@ -1174,16 +1471,17 @@ void run_force_lj_init(State& s, const PendingForce& p, double dt_final, double 
         pa.base = gm == 1 ? 0 : 8;
         for (int d = 0; d < 3; ++d) pa.len[d] = s.geo.len[d];
     }
-    const int nb = nblocks(N + pa.nchain, kThreads);
+    const int lanes = force_lanes(N, s.precision == 1);
+    const int nb = force_blocks(N, lanes, pa.nchain);
     const bool thermo = s.thermo != 0;
     if (thermo) ensure_red_scratch(s, kThermoQ * nb);
     prof_begin(K_FORCE_LJ);
     if (push) {
-        if (thermo) launch_lj<false, true, true, true, true>(s, a, nb, pa);
-        else launch_lj<false, true, false, true, true>(s, a, nb, pa);
+        if (thermo) launch_lj<false, true, true, true, true>(s, a, nb, lanes, pa);
+        else launch_lj<false, true, false, true, true>(s, a, nb, lanes, pa);
     } else {
-        if (thermo) launch_lj<false, true, true, true>(s, a, nb);
-        else launch_lj<false, true, false, true>(s, a, nb);
+        if (thermo) launch_lj<false, true, true, true>(s, a, nb, lanes);
+        else launch_lj<false, true, false, true>(s, a, nb, lanes);
     }
     launched(K_FORCE_LJ);
     prof_end(K_FORCE_LJ);
