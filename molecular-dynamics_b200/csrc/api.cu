@@ -829,6 +829,7 @@ int md_initialize_grid(double const* masses, Vector3D const* positions, Vector3D
     if (s.halo.on) s.ghost_exact = 1;  // ghosts of other ranks are exact images; own ones likewise
     s.pc = s.vc = s.ac = 0;
     s.lists_valid = 0;
+    s.cells_filled = 0;
     s.pend_init = false;
     s.pend_force = PendingForce();
     s.pend_final = s.pend_ghost = s.pend_kick = s.pend_pbc = false;

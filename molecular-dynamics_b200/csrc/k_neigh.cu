@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_count(double4* __rest
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // the binning that follows starts from zeroed cell counters and status (no memsets there)
     for (int g = r; g < nseg; g += gridDim.x * blockDim.x) cnt[g] = 0;
-    if (r == 0) st->out_local = st->out_ghost = st->nchain = st->img_over1 = st->img_over2 = 0;
+    if (r == 0) st->out_local = st->out_ghost = st->nchain = st->img_over1 = st->img_over2 = st->filled = 0;
     unsigned m = 0;
     if (r < N) {
         const int sl = slot_of_ref[r];
@@ -348,18 +348,23 @@ __global__ void k_rank_move(const int* __restrict__ cstart, const int* __restric
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     // the list build that follows starts from a zeroed status (no memset there)
     if (e == 0) st->max_nb = 0;
-    if (e >= NA) return;
-    const int o = tmp_src[e];
-    const int key = tmp_key[e];
-    const int c = m.bin_cell[o];
+    const int o = e < NA ? tmp_src[e] : 0;
+    const int key = e < NA ? tmp_key[e] : 0;
+    const int c = e < NA ? m.bin_cell[o] : ncells;
     int n = e;  // atoms outside the grid keep their bucket order
+    bool first = false;
     if (c != ncells) {
         const int seg = o < m.N ? c : ncells + 1 + c;
         const int a = cstart[seg], b = cstart[seg + 1];
         int rank = 0;
         for (int f = a; f < b; ++f) rank += tmp_key[f] < key;
         n = a + rank;
+        first = rank == 0 && o < m.N;
     }
+    // cells that hold locals (the next list build's choice of kernel)
+    const int filled = __syncthreads_count(first);
+    if (threadIdx.x == 0 && filled) atomicAdd(&st->filled, filled);
+    if (e >= NA) return;
     move_slot(n, o, m, ga);
 }
 
@@ -426,14 +431,23 @@ __device__ __forceinline__ bool exact_within(const double4* __restrict__ pos, in
     return len2_strict(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z)) <= cut2;
 }
 
-// Warp per cell (core/neighborlist.impala:18-78), one home atom per lane (32 at a time).  The
-// 27 stencil cells' candidates (locals then ghosts per cell, stencil order) are staged in shared
-// memory, keeping only those within the list cutoff (with the FP32 margin) of the bounding box
-// of the homes, in order; then every lane walks the kept candidates (one broadcast read each)
-// and appends its own pairs, so each list comes out in stencil order -- the reference's, which
-// fixes the FP64 summation order -- with no cross-lane compaction.  Lanes without a home sit
-// far away and never match.  Pairs near the cutoff take the reference's FP64 test
-// (rsq <= cutoff^2), so membership is exactly the reference's.
+// A block builds the lists of one cell's atoms, the homes, 32 at a time (core/neighborlist.impala:
+// 18-78).  The 27 stencil cells' atoms (locals then ghosts per cell, in stencil order) are staged in
+// shared memory in order, keeping those within the list cutoff (plus the FP32 margin) of the homes'
+// bounding box; then each warp takes every fourth home and tests 32 staged candidates at once, one
+// per lane.  The ballot of the hits gives each hit its place, so a list comes out in stencil order --
+// the reference's, which fixes the FP64 summation order.  A home's entries collect in shared memory
+// and leave as whole quads.  Pairs near the cutoff take the reference's FP64 test (rsq <= cutoff^2),
+// so membership is exactly the reference's; the FP32 margin follows from the magnitude of the staged
+// coordinates (margin32), which makes that test rare.
+//
+// Bound by instruction issue (75 %): 67 M warp instructions at 131,072 atoms, 41 M of them the 1.4 M
+// steps of 32 pair tests, the rest the staging.  One warp per cell with a home per lane walking the
+// candidates one by one, as this kernel did before, took 83 M (19 of 32 lanes held a home) and made
+// small systems wait for one serial walk.  Measured before -> now (us): 256 atoms 43 -> 15, 2,048
+// 48 -> 18, 16,384 51 -> 23, 131,072 124 -> 91, 442,368 336 -> 268; half lists at 131,072 167 -> 102.
+// A step of 1, 3 or 4 chunks instead of 2: 97, 92, 96 us at 131,072; the FP64 test or the emptying of
+// a full buffer inside the step loop, where the compiler predicates it: 130 us.
 //
 // List layout: quads of four consecutive entries of one atom, atom-fastest (nl_index): a force
 // kernel reads four entries with one 16-byte load, and the quads of a warp's 32 atoms form one
@@ -441,57 +455,121 @@ __device__ __forceinline__ bool exact_within(const double4* __restrict__ pos, in
 // rebasing cell minus the home's (mixed form).  A list's last quad is padded with the home
 // itself one rebasing cell away on every axis (code 42), which every force kernel skips by
 // count or finds beyond its cutoff.
-#ifndef TMD_NL_WARPS
-#define TMD_NL_WARPS 4
-#endif
-#ifndef TMD_NL_TILE
-#define TMD_NL_TILE 128
-#endif
-#ifndef TMD_NL_MINB
-#define TMD_NL_MINB 8  // 64 registers: eight blocks of four warps per SM
-#endif
-#ifndef TMD_NL_UNROLL
-#define TMD_NL_UNROLL 4
-#endif
-constexpr int kNlWarps = TMD_NL_WARPS;    // warps (cells) per block
-constexpr int kNlTile = TMD_NL_TILE;      // kept candidates staged per warp before the homes walk them
-constexpr int kNlUnroll = TMD_NL_UNROLL;  // candidates per step of a home's walk
-constexpr uint32_t kPadCode = 42u;        // dk = +1 on every axis
+constexpr int kNlThreads = 128, kNlWarps = kNlThreads / 32;
+constexpr int kNlChunks = 5;                // candidates staged per lane and tile
+constexpr int kNlTile = kNlThreads * kNlChunks;  // candidates staged at once
+constexpr int kNlStep = 2;                  // chunks of 32 candidates a home tests at once
+constexpr int kNlBuf = 128 + 32 * kNlStep;  // entries of a home collected before they leave as quads
+constexpr uint32_t kPadCode = 42u;          // dk = +1 on every axis
 
 struct NlArgs {
-    double cut2;     // cutoff^2 (FP64, the reference's membership test)
-    float lo2, hi2;  // FP32 prefilter: certainly inside below lo2, certainly outside above hi2
+    double cut2;  // cutoff^2 (FP64, the reference's membership test)
+    float cut;
     int nbcap, stride, N, ncells, nx, nxy;
     double alo[3], spacing;
 };
 
-template <int HM, typename IDX>
-__global__ void __launch_bounds__(kNlWarps * 32, TMD_NL_MINB)
+// Bound of |r^2 (FP32) - r^2 (exact)| for a pair near the cutoff whose staged coordinates are at
+// most `mag` in magnitude: each coordinate is rounded once (2^-24 mag) and so is each difference
+// (2^-24 cut), an error of del below 3 * 2^-24 mag per axis, of r^2 below 2 sqrt(3) cut times that
+// plus 3 roundings of r^2; three times that sum is taken.
+__device__ __forceinline__ float margin32(float cut, float mag) {
+    constexpr float u = 1.0f / 16777216.0f;
+    return 3.0f * (10.4f * u * cut * fmaxf(mag, cut) + 3.0f * u * cut * cut);
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+    asm("redux.sync.min.f32 %0, %0, 0xffffffff;" : "+f"(v));
+    return v;
+}
+
+// shared memory by its 32-bit address (the walk's inner loop steps addresses, not indices)
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float4 lds_f4(uint32_t p) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p));
+    return v;
+}
+__device__ __forceinline__ int lds_i(uint32_t p) {
+    int v;
+    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(p));
+    return v;
+}
+__device__ __forceinline__ void sts_u(uint32_t p, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+}
+
+// writes the quads of buf[0, n) (n a multiple of four) to the list of atom i from entry k0 on
+__device__ __forceinline__ void store_quads(const uint32_t* buf, int n, int k0, int i, uint32_t* __restrict__ nbl,
+                                            const NlArgs& a, int lane) {
+    for (int q = lane; 4 * q < n; q += 32)
+        if (k0 + 4 * q < a.nbcap)
+            reinterpret_cast<uint4*>(nbl)[(size_t)((k0 >> 2) + q) * a.stride + i] =
+                reinterpret_cast<const uint4*>(buf)[q];
+}
+
+// the buffer holds 128 entries or more: 32 whole quads leave and the rest moves up; a later tile's
+// list that starts inside a quad leaves entry by entry
+__device__ __forceinline__ void drain(uint32_t* buf, int& nb, int& out, int i, uint32_t* __restrict__ nbl,
+                                   const NlArgs& a, int lane) {
+    __syncwarp();
+    if ((out & 3) == 0) {
+        store_quads(buf, 128, out, i, nbl, a, lane);
+        nb -= 128;
+        out += 128;
+        uint32_t rest[kNlStep];
+#pragma unroll
+        for (int u = 0; u < kNlStep; ++u) rest[u] = buf[128 + 32 * u + lane];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kNlStep; ++u)
+            if (32 * u + lane < nb) buf[32 * u + lane] = rest[u];
+    } else {
+        for (int e = lane; e < nb; e += 32)
+            if (out + e < a.nbcap) nbl[nl_index(out + e, i, a.stride)] = buf[e];
+        out += nb;
+        nb = 0;
+        __syncwarp();
+    }
+}
+
+template <int HM>
+__global__ void __launch_bounds__(kNlThreads, 8)
 k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const int* __restrict__ rbk,
              const int* __restrict__ cstart, int* __restrict__ nbn, uint32_t* __restrict__ nbl, DevStatus* st,
              NlArgs a, int cell_blocks, LinkArgs la) {
-    // kept candidate position (cell-centre relative); w = slot << 6 + its rebasing cell relative to
-    // the first home's (rel_code) + kCodeBias, from which a home's entry is one subtraction
-    __shared__ float4 s_cpos[kNlWarps][kNlTile];
-    __shared__ int s_cref[kNlWarps][HM ? kNlTile : 1];
-    __shared__ int s_rstart[kNlWarps][54];
-    __shared__ int s_rpre[kNlWarps][55];
+    // candidate position (cell-centre relative); w = slot << 6 + its rebasing cell relative to the
+    // first home's (rel_code) + kCodeBias, from which a home's entry is one subtraction
+    __shared__ float4 s_cand[kNlTile + 32 * kNlStep];
+    __shared__ int s_cref[HM ? kNlTile + 32 * kNlStep : 1];
+    __shared__ float4 s_home[32];  // position; w = its relative rebasing cell
+    __shared__ int s_href[HM ? 32 : 1];
+    __shared__ int s_cnt[32];      // entries of each home so far (cells of more than one tile)
+    __shared__ int s_rstart[54];   // the stencil's ranges: first slot, candidates before it
+    __shared__ int s_rpre[55];
+    __shared__ int s_nr;
+    __shared__ int s_slot[kNlTile];  // slots of the tile's candidates
+    __shared__ float4 s_box[2];    // the homes' bounding box; w = r^2 certainly inside, outside
+    __shared__ double s_ctr[3];    // the cell's centre
+    __shared__ int s_rb0;          // the first home's rebasing cell
+    __shared__ int s_kept[kNlWarps];
+    __shared__ __align__(16) uint32_t s_buf[kNlThreads / 32][kNlBuf];
 
-    if (blockIdx.x >= cell_blocks) {  // blocks past the cells link the ghosts (k_ghost_links' work)
+    if ((int)blockIdx.x >= cell_blocks) {  // blocks past the cells link the ghosts (k_ghost_links' work)
         const int h = (blockIdx.x - cell_blocks) * blockDim.x + threadIdx.x;
         if (h < la.G) ghost_link(h, la);
         return;
     }
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x * kNlWarps + wid;
-    if (c >= a.ncells) return;
+    const int c = blockIdx.x;
     const int h0 = cstart[c], h1 = cstart[c + 1];
     if (h0 == h1) return;
     const unsigned lt = lanemask_lt();
 
-    // 27 stencil cells in the reference order (z, y, x offsets -1..1), each contributing
-    // its locals then its ghosts (54 ranges); lane l owns ranges 2l and 2l + 1
-    {
+    // 27 stencil cells in the reference order (z, y, x offsets -1..1), each contributing its locals
+    // then its ghosts: 54 ranges of slots.  Without ghosts around, the three cells of an x row are one
+    // range: 9 ranges.  One warp of the group finds them while another looks at the homes.
+    if (wid == 0) {
         int start = 0, len = 0, gs = 0, gl = 0;
         if (lane < 27) {
             const int oz = lane / 9 - 1, oy = (lane / 3) % 3 - 1, ox = lane % 3 - 1;
@@ -503,138 +581,367 @@ k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const
                 gl = cstart[a.ncells + 2 + nb] - gs;
             }
         }
+        const bool ghosts = __any_sync(0xffffffffu, gl > 0);
         int incl = len + gl;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        if (lane < 27) {
-            const int ex = incl - len - gl;
-            s_rstart[wid][2 * lane] = start;
-            s_rstart[wid][2 * lane + 1] = gs;
-            s_rpre[wid][2 * lane] = ex;
-            s_rpre[wid][2 * lane + 1] = ex + len;
+        const int ex = incl - len - gl;
+        if (ghosts) {
+            if (lane < 27) {
+                s_rstart[2 * lane] = start;
+                s_rstart[2 * lane + 1] = gs;
+                s_rpre[2 * lane] = ex;
+                s_rpre[2 * lane + 1] = ex + len;
+            }
+        } else {
+            // a row's start is its first cell with atoms
+            const int l1 = __shfl_down_sync(0xffffffffu, len, 1);
+            const int s1 = __shfl_down_sync(0xffffffffu, start, 1), s2 = __shfl_down_sync(0xffffffffu, start, 2);
+            if (lane < 27 && lane % 3 == 0) {
+                s_rstart[lane / 3] = len ? start : (l1 ? s1 : s2);
+                s_rpre[lane / 3] = ex;
+            }
         }
-        if (lane == 26) s_rpre[wid][54] = incl;
+        if (lane == 26) {
+            s_rpre[ghosts ? 54 : 9] = incl;
+            s_nr = ghosts ? 54 : 9;
+        }
     }
-    __syncwarp();
-    const int M = s_rpre[wid][54];
 
-    const int cz = c / a.nxy, cy = (c / a.nx) % (a.nxy / a.nx), cx = c % a.nx;
-    const double ctr[3] = {a.alo[0] + ((double)cx + 0.5) * a.spacing, a.alo[1] + ((double)cy + 0.5) * a.spacing,
-                           a.alo[2] + ((double)cz + 0.5) * a.spacing};
-    const int rb0 = __ldg(rbk + h0);  // rebasing cells are staged relative to the first home's
+    uint32_t* buf = s_buf[wid];
     int maxcnt = 0;
 
     for (int hb = h0; hb < h1; hb += 32) {
         const int hn = min(32, h1 - hb);
-        const bool home = lane < hn;
-        const int i = hb + (home ? lane : 0);
-        float hx = 1e18f, hy = 1e18f, hz = 1e18f;  // no home: never within the cutoff
-        int irel = 0, iref = 0;
-        if (home) {
-            const double4 p = pos[i];
-            hx = (float)(p.x - ctr[0]);
-            hy = (float)(p.y - ctr[1]);
-            hz = (float)(p.z - ctr[2]);
-            irel = rel_code(rbk[i], rb0);
-            if (HM) iref = ref[i];
+        if (hb > h0) __syncthreads();  // every warp has left the previous homes
+        if (wid == kNlWarps - 1) {
+            // the homes and their bounding box, relative to the cell's centre
+            const bool home = lane < hn;
+            const int i = hb + (home ? lane : 0);
+            const double4 p = ldg_d4(pos + i);
+            const int rb = __ldg(rbk + i), rb0 = __ldg(rbk + h0);
+            const int cz = c / a.nxy, cy = (c - cz * a.nxy) / a.nx, cx = c - cz * a.nxy - cy * a.nx;
+            const double ox = a.alo[0] + ((double)cx + 0.5) * a.spacing, oy = a.alo[1] + ((double)cy + 0.5) * a.spacing,
+                         oz = a.alo[2] + ((double)cz + 0.5) * a.spacing;
+            const float hx = (float)(p.x - ox), hy = (float)(p.y - oy), hz = (float)(p.z - oz);
+            if (home) {
+                s_home[lane] = make_float4(hx, hy, hz, __int_as_float(rel_code(rb, rb0)));
+                if (HM) s_href[lane] = __ldg(ref + i);
+                s_cnt[lane] = 0;
+            }
+            const float lx = warp_min(hx), ly = warp_min(hy), lz = warp_min(hz);
+            const float ux = -warp_min(-hx), uy = -warp_min(-hy), uz = -warp_min(-hz);
+            if (lane == 0) {
+                const float mag = fmaxf(fmaxf(fmaxf(-lx, ux), fmaxf(-ly, uy)), fmaxf(-lz, uz)) + a.cut;
+                const float margin = margin32(a.cut, mag), cut2 = a.cut * a.cut;
+                s_box[0] = make_float4(lx, ly, lz, cut2 - margin);
+                s_box[1] = make_float4(ux, uy, uz, cut2 + margin);
+                s_ctr[0] = ox;
+                s_ctr[1] = oy;
+                s_ctr[2] = oz;
+                s_rb0 = rb0;
+            }
         }
-        // a candidate's staged w minus irel is the entry slot << 6 | code; it equals i6 only for
-        // the home itself (within the cutoff the two rebasing parts differ by less than 64)
-        const uint32_t i6 = ((uint32_t)i << kCodeBits) + (uint32_t)(irel + kCodeBias);
-        // nl_index in the list's index type: 32-bit unless the list holds 2^32 entries or more
-        // (the 64-bit index arithmetic made the build 15 % slower)
-        const IDX i4 = HM ? 0 : (IDX)i * 4u, stride4 = HM ? 0 : (IDX)a.stride * 4u;  // (the half lists: nl_index)
-        // bounding box of the homes, widened by the list cutoff (with the FP32 margin)
-        float lo[3] = {home ? hx : INFINITY, home ? hy : INFINITY, home ? hz : INFINITY};
-        float hi[3] = {home ? hx : -INFINITY, home ? hy : -INFINITY, home ? hz : -INFINITY};
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], off));
-                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], off));
+        __syncthreads();  // ranges and homes are in place
+        const int nr = s_nr, M = s_rpre[nr];
+
+        for (int t0 = 0; t0 < M; t0 += kNlTile) {
+            // the slots of the tile's candidates, range by range
+            const int t1 = min(t0 + kNlTile, M);
+            for (int r = wid; r < nr; r += kNlWarps) {
+                const int first = s_rpre[r], m1 = min(s_rpre[r + 1], t1);
+                const int slot = s_rstart[r] - first;
+                for (int m = max(first, t0) + lane; m < m1; m += 32) s_slot[m - t0] = slot + m;
             }
-        int cnt = 0;
-        int t0 = 0;  // next candidate to stage (M > 0: the home cell is in the stencil)
-        do {
-            int nk = 0;  // kept candidates staged (warp-uniform)
-            // stage: keep candidates in order until the next chunk might not fit
-            while (t0 < M && nk + 32 <= kNlTile) {
-                const int m = t0 + lane;
-                bool keep = false;
-                float4 cp;
-                int cref = 0;
-                if (m < M) {
-                    int lo_r = 0, hi_r = 53;  // the range of candidate m: the last one starting at or before m
-                    while (lo_r < hi_r) {
-                        const int mid = (lo_r + hi_r + 1) >> 1;
-                        if (s_rpre[wid][mid] <= m) lo_r = mid;
-                        else hi_r = mid - 1;
+            __syncthreads();
+            // this warp's share of the tile, a whole number of chunks, kept in registers until the
+            // warps before it know how many they keep
+            const int share = ((t1 - t0 + kNlThreads - 1) / kNlThreads) * 32;
+            const int m0 = wid * share, m1 = min(m0 + share, t1 - t0);
+            const float4 lo = s_box[0], hi = s_box[1];
+            const double ox = s_ctr[0], oy = s_ctr[1], oz = s_ctr[2];
+            const int rb0 = s_rb0;  // rebasing cells are staged relative to the first home's
+            float4 cp[kNlChunks];
+            int cref[HM ? kNlChunks : 1];
+            unsigned bal[kNlChunks];
+            int kept = 0;
+#pragma unroll
+            for (int u = 0; u < kNlChunks; ++u) {
+                bal[u] = 0u;
+                if (m0 + 32 * u >= m1) continue;  // warp-uniform
+                const int m = m0 + 32 * u + lane;
+                const int slot = s_slot[min(m, m1 - 1)];
+                const double4 p = ldg_d4(pos + slot);
+                const int kb = __ldg(rbk + slot);
+                if (HM) cref[u] = __ldg(ref + slot);  // root reference index (ref for locals)
+                cp[u] = make_float4((float)(p.x - ox), (float)(p.y - oy), (float)(p.z - oz),
+                                    __uint_as_float(((uint32_t)slot << kCodeBits) +
+                                                    (uint32_t)(rel_code(kb, rb0) + kCodeBias)));
+                const float ex = fmaxf(fmaxf(lo.x - cp[u].x, cp[u].x - hi.x), 0.f);
+                const float ey = fmaxf(fmaxf(lo.y - cp[u].y, cp[u].y - hi.y), 0.f);
+                const float ez = fmaxf(fmaxf(lo.z - cp[u].z, cp[u].z - hi.z), 0.f);
+                bal[u] = __ballot_sync(0xffffffffu, m < m1 && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= hi.w);
+                kept += __popc(bal[u]);
+            }
+            if (lane == 0) s_kept[wid] = kept;
+            __syncthreads();  // the shares are known, and every warp has left the previous tile
+            int at = 0, nk = 0;
+#pragma unroll
+            for (int w = 0; w < kNlWarps; ++w) {
+                const int kw = s_kept[w];
+                at += w < wid ? kw : 0;
+                nk += kw;
+            }
+#pragma unroll
+            for (int u = 0; u < kNlChunks; ++u) {
+                if ((bal[u] >> lane) & 1u) {
+                    const int k = at + __popc(bal[u] & lt);
+                    s_cand[k] = cp[u];
+                    if (HM) s_cref[k] = cref[u];
+                }
+                at += __popc(bal[u]);
+            }
+            if (wid == kNlWarps - 1) {  // the last step filled up with candidates that nothing is near
+#pragma unroll
+                for (int u = 0; u < kNlStep; ++u) {
+                    s_cand[nk + 32 * u + lane] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+                    if (HM) s_cref[nk + 32 * u + lane] = 0x7fffffff;
+                }
+            }
+            __syncthreads();
+
+            const bool last = t1 == M;
+            const float lo2 = lo.w, hi2 = hi.w;
+            const uint32_t cand0 = smem_addr(&s_cand[lane]), cand_end = smem_addr(&s_cand[0]) + 16 * nk + 16 * lane;
+            const uint32_t cref0 = smem_addr(&s_cref[HM ? lane : 0]);
+            const uint32_t buf0 = smem_addr(buf), buf_full = buf0 + 4 * 128;
+            for (int h = wid; h < hn; h += kNlWarps) {
+                const float4 hp = s_home[h];
+                const int i = hb + h;
+                const uint32_t irel = __float_as_uint(hp.w);
+                // a candidate's staged w minus irel is the entry slot << 6 | code; it equals i6 only
+                // for the home itself (within the cutoff the two rebasing parts differ by less than 64)
+                const uint32_t i6 = ((uint32_t)i << kCodeBits) + (uint32_t)((int)irel + kCodeBias);
+                const int iref = HM ? s_href[HM ? h : 0] : 0;
+                int out = M > kNlTile ? s_cnt[h] : 0;  // entries already in the list
+                uint32_t bp = buf0;                       // where the next entry goes in the buffer
+                uint32_t cp0 = cand0, cr0 = cref0;        // the lane's candidate of this step
+                for (;;) {
+                    bool take[kNlStep], near = false, may[kNlStep], slow;
+                    uint32_t entry[kNlStep];
+                    for (; cp0 < cand_end; cp0 += 512 * kNlStep, cr0 += 128 * kNlStep) {
+                        near = bp >= buf_full;
+#pragma unroll
+                        for (int u = 0; u < kNlStep; ++u) {
+                            const float4 q = lds_f4(cp0 + 512 * u);
+                            const float dx = hp.x - q.x, dy = hp.y - q.y, dz = hp.z - q.z;
+                            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                            const uint32_t s6 = __float_as_uint(q.w);
+                            // the entry slot << 6 | code: the list cutoff below the rebasing spacing
+                            // keeps every |dk| <= 1 within it (checked on the host)
+                            entry[u] = s6 - irel;
+                            // core/neighborlist.impala:34: half lists keep i > j (reference index); HM ==
+                            // 2 compares ghosts by their root so pairs across the periodic boundary are
+                            // kept once
+                            may[u] = s6 != i6 && (!HM || lds_i(cr0 + 128 * u) < iref);
+                            const bool in = r2 < lo2;
+                            take[u] = may[u] && in;
+                            near = near || (!in && r2 <= hi2);
+                        }
+                        slow = __any_sync(0xffffffffu, near);
+                        if (slow) break;
+#pragma unroll
+                        for (int u = 0; u < kNlStep; ++u) {
+                            const unsigned hits = __ballot_sync(0xffffffffu, take[u]);
+                            if (take[u]) sts_u(bp + 4 * __popc(hits & lt), entry[u]);
+                            bp += 4 * __popc(hits);
+                        }
                     }
-                    const int slot = s_rstart[wid][lo_r] + (m - s_rpre[wid][lo_r]);
-                    // the candidate's position, rebasing cell and key load together (one latency)
-                    const double4 p = pos[slot];
-                    const int kb = __ldg(rbk + slot);
-                    if (HM) cref = __ldg(ref + slot);  // root reference index (ref for locals)
-                    cp = make_float4((float)(p.x - ctr[0]), (float)(p.y - ctr[1]), (float)(p.z - ctr[2]),
-                                     __uint_as_float(((uint32_t)slot << kCodeBits) +
-                                                     (uint32_t)(rel_code(kb, rb0) + kCodeBias)));
-                    const float ex = fmaxf(fmaxf(lo[0] - cp.x, cp.x - hi[0]), 0.f);
-                    const float ey = fmaxf(fmaxf(lo[1] - cp.y, cp.y - hi[1]), 0.f);
-                    const float ez = fmaxf(fmaxf(lo[2] - cp.z, cp.z - hi[2]), 0.f);
-                    keep = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= a.hi2;
+                    if (cp0 >= cand_end) break;
+                    // a step with a pair near the cutoff, or a full buffer (kept out of the loop above,
+                    // where the compiler would run all of this predicated on every step)
+                    if (bp >= buf_full) {
+                        int nb = (int)(bp - buf0) >> 2;
+                        drain(buf, nb, out, i, nbl, a, lane);
+                        bp = buf0 + 4 * nb;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kNlStep; ++u) {
+                        const float4 q = lds_f4(cp0 + 512 * u);
+                        const float dx = hp.x - q.x, dy = hp.y - q.y, dz = hp.z - q.z;
+                        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                        bool in = r2 < lo2;
+                        // |dk| <= 1 still holds near the cutoff, so the entry's slot is the candidate's
+                        if (may[u] && !in && r2 <= hi2)
+                            in = exact_within(pos, i, (int)(entry[u] >> kCodeBits), a.cut2);
+                        const bool t = may[u] && in;
+                        const unsigned hits = __ballot_sync(0xffffffffu, t);
+                        if (t) sts_u(bp + 4 * __popc(hits & lt), entry[u]);
+                        bp += 4 * __popc(hits);
+                    }
+                    cp0 += 512 * kNlStep;
+                    cr0 += 128 * kNlStep;
                 }
-                const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const int at = nk + __popc(bal & lt);
-                    s_cpos[wid][at] = cp;
-                    if (HM) s_cref[wid][at] = cref;
+                int nb = (int)(bp - buf0) >> 2;  // entries in the buffer
+                if (nb >= 128) drain(buf, nb, out, i, nbl, a, lane);
+                __syncwarp();
+                if ((out & 3) == 0 && last) {
+                    // the last quad's padding
+                    if (lane < ((-nb) & 3)) buf[nb + lane] = ((uint32_t)i << kCodeBits) | kPadCode;
+                    __syncwarp();
+                    store_quads(buf, (nb + 3) & ~3, out, i, nbl, a, lane);
+                } else {
+                    for (int e = lane; e < nb; e += 32)
+                        if (out + e < a.nbcap) nbl[nl_index(out + e, i, a.stride)] = buf[e];
+                    if (last && lane < ((-(out + nb)) & 3) && out + nb + lane < a.nbcap)
+                        nbl[nl_index(out + nb + lane, i, a.stride)] = ((uint32_t)i << kCodeBits) | kPadCode;
                 }
-                nk += __popc(bal);
-                t0 += 32;
+                __syncwarp();  // the buffer is free for the next home
+                const int cnt = out + nb;
+                if (last) {
+                    if (lane == 0) nbn[i] = cnt;
+                    maxcnt = max(maxcnt, cnt);
+                } else if (lane == 0) {
+                    s_cnt[h] = cnt;
+                }
             }
-            __syncwarp();
-            // every home walks the kept candidates in order
-#pragma unroll kNlUnroll
-            for (int k = 0; k < nk; ++k) {
-                const float4 cp = s_cpos[wid][k];
-                const float dx = hx - cp.x, dy = hy - cp.y, dz = hz - cp.z;
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                const uint32_t s6 = __float_as_uint(cp.w);
-                bool in = r2 < a.lo2;
-                // near the cutoff (|dk| <= 1 still holds there): s6 - irel is the entry, its slot the candidate's
-                if (!in && r2 <= a.hi2) in = exact_within(pos, i, (s6 - (uint32_t)irel) >> kCodeBits, a.cut2);
-                // core/neighborlist.impala:34: half lists keep i > j (reference index); HM == 2
-                // compares ghosts by their root so pairs across the periodic boundary are kept once
-                const bool take = in && s6 != i6 && (!HM || s_cref[wid][HM ? k : 0] < iref);
-                // the entry slot << 6 | code: the list cutoff below the rebasing spacing keeps
-                // every |dk| <= 1 within it (checked on the host)
-                if (HM) {
-                    // half lists: the append without a branch (measured faster there, while
-                    // the full-list walk is faster with the branch)
-                    if (take && cnt < a.nbcap) nbl[nl_index(cnt, i, a.stride)] = s6 - (uint32_t)irel;
-                    cnt += take ? 1 : 0;
-                } else if (take) {
-                    // (a store at every step, without the branch: 147 -> 182 us at 131k atoms)
-                    if (cnt < a.nbcap) nbl[(IDX)(cnt >> 2) * stride4 + i4 + (IDX)(cnt & 3)] = s6 - (uint32_t)irel;
-                    ++cnt;
-                }
-            }
-            __syncwarp();
-        } while (t0 < M);
-        if (home) {
-            nbn[i] = cnt;
-            // the last quad's padding
-            const uint32_t pad = ((uint32_t)i << kCodeBits) | kPadCode;
-            for (int q = cnt; (q & 3) != 0 && q < a.nbcap; ++q) nbl[nl_index(q, i, a.stride)] = pad;
-            maxcnt = max(maxcnt, cnt);
         }
     }
-    maxcnt = warp_max(maxcnt);
-    if (lane == 0) atomicMax(&st->max_nb, maxcnt);
+    if (lane == 0 && maxcnt > 0) atomicMax(&st->max_nb, maxcnt);
+}
+
+// Sparse cells (DEM grains: ~3 to a cell and ~90 in its stencil): eight lanes to a home, four homes
+// to a warp.  A home's lanes lay its stencil's ranges of slots end to end (9 rows, or 54 ranges where
+// ghosts are around) and test eight candidates at once with the reference's FP64 test; the ballot
+// among them places the hits.  Bound by instruction issue and
+// latency (65 %, ~1,000 warp instructions per four homes).  The kernel above gives each cell a block,
+// most of it idle here: contact DEM, before (a warp per cell) -> now, us: 260,800 grains 187 -> 86,
+// 223,488 162 -> 79, 33,000 35 -> 21.  A thread per home took 88, 101 and 53 us; ballots among the
+// eight lanes alone instead of the whole warp 106, 94 and 25 us.
+constexpr int kSparseThreads = 128, kSparseLanes = 8;
+constexpr int kSparseBatch = 2;  // candidates of a lane in flight (4: 95 us at 260,800 grains)
+
+template <int HM>
+__global__ void __launch_bounds__(kSparseThreads)
+k_build_list_sparse(const double4* __restrict__ pos, const int* __restrict__ ref, const int* __restrict__ rbk,
+                    const int* __restrict__ cstart, const int* __restrict__ slot_cell, int* __restrict__ nbn,
+                    uint32_t* __restrict__ nbl, DevStatus* st, NlArgs a, int local_blocks, LinkArgs la) {
+    // a home's ranges: candidates before it, first slot minus that
+    __shared__ int2 s_range[kSparseThreads / kSparseLanes][55];
+    if ((int)blockIdx.x >= local_blocks) {  // blocks past the locals link the ghosts (k_ghost_links' work)
+        const int h = (blockIdx.x - local_blocks) * blockDim.x + threadIdx.x;
+        if (h < la.G) ghost_link(h, la);
+        return;
+    }
+    const int lane = threadIdx.x & 31, l = lane % kSparseLanes;
+    const int i = (blockIdx.x * kSparseThreads + threadIdx.x) / kSparseLanes;
+    const unsigned group = 0xffu << (lane - l), before = lanemask_lt() & group;
+    int cnt = 0;
+    // a home outside the grid (or past the last one) has no candidates; the warp's homes keep together,
+    // so that shuffles and ballots run over whole warps
+    const int c = i < a.N ? slot_cell[i] : a.ncells;
+    const bool act = c < a.ncells;
+    const int ih = act ? i : 0;
+    const double4 pi = ldg_d4(pos + ih);
+    const int rb = __ldg(rbk + ih);
+    const int iref = HM ? __ldg(ref + ih) : 0;
+    const int* gstart = cstart + a.ncells + 1;
+    int2* range = s_range[threadIdx.x / kSparseLanes];
+    // lane l takes row l of the stencil, all lanes row 8
+    int len[2], start[2];
+    bool ghosts = false;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int r = q ? 8 : l;
+        const int row = c + (r / 3 - 1) * a.nxy + (r % 3 - 1) * a.nx;
+        const int c0 = min(max(row - 1, 0), a.ncells), c1 = act ? min(max(row + 2, 0), a.ncells) : c0;
+        start[q] = __ldg(cstart + c0);
+        len[q] = __ldg(cstart + c1) - start[q];
+        ghosts = ghosts || __ldg(gstart + c0) != __ldg(gstart + c1);
+    }
+    int M;
+    if (!__any_sync(0xffffffffu, ghosts)) {
+        int incl = len[0];
+#pragma unroll
+        for (int o = 1; o < kSparseLanes; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o, kSparseLanes);
+            if (l >= o) incl += y;
+        }
+        range[l] = make_int2(incl - len[0], start[0] - (incl - len[0]));
+        if (l == kSparseLanes - 1) range[8] = make_int2(incl, start[1] - incl);
+        M = __shfl_sync(0xffffffffu, incl, kSparseLanes - 1, kSparseLanes) + len[1];
+        if (l == 0) range[9] = make_int2(M, 0);
+    } else {  // cell by cell, the locals then the ghosts of each
+        M = 0;
+        for (int k0 = 0; k0 < 27; k0 += kSparseLanes) {
+            const int k = k0 + l, nb = c + (k / 9 - 1) * a.nxy + ((k / 3) % 3 - 1) * a.nx + k % 3 - 1;
+            int ls = 0, ll = 0, gs = 0, gl = 0;
+            if (act && k < 27 && nb >= 0 && nb < a.ncells) {
+                ls = __ldg(cstart + nb);
+                ll = __ldg(cstart + nb + 1) - ls;
+                gs = __ldg(gstart + nb);
+                gl = __ldg(gstart + nb + 1) - gs;
+            }
+            int incl = ll + gl;
+#pragma unroll
+            for (int o = 1; o < kSparseLanes; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o, kSparseLanes);
+                if (l >= o) incl += y;
+            }
+            const int ex = M + incl - ll - gl;
+            if (k < 27) {
+                range[2 * k] = make_int2(ex, ls - ex);
+                range[2 * k + 1] = make_int2(ex + ll, gs - ex - ll);
+            }
+            M += __shfl_sync(0xffffffffu, incl, kSparseLanes - 1, kSparseLanes);
+        }
+        if (l == 0) range[54] = make_int2(M, 0);
+    }
+    __syncwarp();
+    const int most = __reduce_max_sync(0xffffffffu, M);
+    int r = 0, rend = range[1].x, roff = range[0].y;
+    for (int m0 = l; m0 - l < most; m0 += kSparseLanes * kSparseBatch) {
+        // positions, rebasing cells and keys of a batch load together
+        double4 p[kSparseBatch];
+        int slot[kSparseBatch], kb[kSparseBatch], kr[HM ? kSparseBatch : 1];
+#pragma unroll
+        for (int u = 0; u < kSparseBatch; ++u) {
+            const int m = m0 + u * kSparseLanes;
+            if (m < M) {
+                while (rend <= m) {
+                    ++r;
+                    rend = range[r + 1].x;
+                    roff = range[r].y;
+                }
+            }
+            slot[u] = m < M ? m + roff : ih;
+            p[u] = ldg_d4(pos + slot[u]);
+            kb[u] = __ldg(rbk + slot[u]);
+            if (HM) kr[u] = __ldg(ref + slot[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kSparseBatch; ++u) {
+            const double r2 = len2_strict(dsub(pi.x, p[u].x), dsub(pi.y, p[u].y), dsub(pi.z, p[u].z));
+            // core/neighborlist.impala:34: half lists keep i > j (reference index); HM == 2 compares
+            // ghosts by their root
+            const bool take = r2 <= a.cut2 && slot[u] != ih && (!HM || kr[HM ? u : 0] < iref);
+            const unsigned hits = __ballot_sync(0xffffffffu, take) & group;
+            const int k = cnt + __popc(hits & before);
+            if (take && k < a.nbcap)
+                nbl[nl_index(k, i, a.stride)] =
+                    ((uint32_t)slot[u] << kCodeBits) + (uint32_t)(rel_code(kb[u], rb) + kCodeBias);
+            cnt += __popc(hits);
+        }
+    }
+    // the last quad's padding
+    if (act && l < ((-cnt) & 3) && cnt + l < a.nbcap)
+        nbl[nl_index(cnt + l, i, a.stride)] = ((uint32_t)i << kCodeBits) | kPadCode;
+    if (i < a.N && l == 0) nbn[i] = cnt;
+    cnt = warp_max(cnt);
+    if (lane == 0 && cnt > 0) atomicMax(&st->max_nb, cnt);
 }
 
 // Locals outside the grid (bucket ncells) get empty lists.
@@ -998,7 +1305,7 @@ void run_distribute(State& s) {
     prof_begin(K_BIN);
     if (!s.bin_zeroed) {  // else zeroed by the border pass's first kernel
         TMD_CUDA(cudaMemsetAsync(s.cnt, 0, sizeof(int) * nseg, s.stream));
-        TMD_CUDA(cudaMemsetAsync(&s.status_dev->out_local, 0, 5 * sizeof(int), s.stream));  // .. img_over2
+        TMD_CUDA(cudaMemsetAsync(&s.status_dev->out_local, 0, 6 * sizeof(int), s.stream));  // .. filled
     }
     s.bin_zeroed = false;
     k_bin_count<<<nblocks(NA, 256), 256, 0, s.stream>>>(s.pos.b[s.pc], s.cnt, s.bin_cell, s.bin_rank, s.status_dev,
@@ -1066,14 +1373,30 @@ void flush_links(State& s) {
     launched(K_BIN);
 }
 
+// Which list kernel: a block per cell from 8.5 locals per filled cell on.  Measured on LJ liquids of
+// 131,072 atoms with smaller cutoffs, block per cell / eight lanes per home, us: 2.8 per cell 158 / 53,
+// 4.9 112 / 69, 7.8 94 / 87, 11.7 85 / 112, 18.5 91 / 158; the same line at 16,384 and 442,368 atoms.
+// Below 4,096 locals the block per cell is as fast or faster at every density.  The filled cells are
+// those of the last binning whose status was read (the results are the same either way); before the
+// first one the box's mean density stands in.
+static bool sparse_cells(const State& s) {
+    const Geometry& g = s.geo;
+    if (s.N <= 4096) return false;
+    if (s.cells_filled > 0) return (double)s.N < 8.5 * s.cells_filled;
+    return (double)s.N * g.spacing * g.spacing * g.spacing < 8.5 * g.len[0] * g.len[1] * g.len[2];
+}
+
 template <int HM>
-void launch_build_list(State& s, bool wide, int blocks, const int* ref, const NlArgs& a, int nb, const LinkArgs& la) {
-    if (wide)
-        k_build_list<HM, size_t><<<blocks, kNlWarps * 32, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart, s.nbn,
-                                                                         s.nbl, s.status_dev, a, nb, la);
-    else
-        k_build_list<HM, uint32_t><<<blocks, kNlWarps * 32, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart,
-                                                                           s.nbn, s.nbl, s.status_dev, a, nb, la);
+void launch_build_list(State& s, const int* ref, const NlArgs& a, const LinkArgs& la, int links) {
+    const int lb = nblocks(links, kNlThreads);
+    if (sparse_cells(s)) {
+        const int nb = nblocks((long long)s.N * kSparseLanes, kSparseThreads);
+        k_build_list_sparse<HM><<<nb + lb, kSparseThreads, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart, s.slot_cell,
+                                                                          s.nbn, s.nbl, s.status_dev, a, nb, la);
+    } else {
+        k_build_list<HM><<<a.ncells + lb, kNlThreads, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart, s.nbn, s.nbl,
+                                                                     s.status_dev, a, a.ncells, la);
+    }
 }
 
 // A list build's status, read back: the locals outside the grid get empty lists, the two-phase
@@ -1091,6 +1414,7 @@ static int finish_build(State& s, bool half) {
         set_error(5, "locals outside the cell grid at binning (they have no neighbours)");
     }
     s.nchain = s.status_host->nchain;
+    s.cells_filled = s.status_host->filled;
     s.img_ok = (s.status_host->img_over1 == 0 ? 1 : 0) | (s.status_host->img_over2 == 0 ? 2 : 0);
     const int mx = s.status_host->max_nb;
     if (mx <= s.nb_cap) {
@@ -1118,9 +1442,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     if (half && s.half_ghost) flush_links(s);
     NlArgs a;
     a.cut2 = cutoff * cutoff;
-    const double margin = 1e-3 * a.cut2 + 1e-6;
-    a.lo2 = (float)(a.cut2 - margin);
-    a.hi2 = (float)(a.cut2 + margin);
+    a.cut = (float)cutoff;
     a.N = s.N;
     a.ncells = g.ncells;
     a.nx = g.nx;
@@ -1128,7 +1450,6 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     a.stride = s.nb_stride;
     for (int d = 0; d < 3; ++d) a.alo[d] = g.aabb_lo[d];
     a.spacing = g.spacing;
-    const int nb = nblocks(g.ncells, kNlWarps);
     for (int attempt = 0; attempt < 8; ++attempt) {
         a.nbcap = s.nb_cap;
         if (attempt > 0 || !s.build_zeroed)  // else zeroed by the binning's reorder kernel
@@ -1137,15 +1458,11 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
         prof_begin(K_NLIST);
         // the pending ghost links ride along as extra blocks (once: they count with atomics)
         const LinkArgs la = link_args(s);
-        const int lb = s.pend_links ? nblocks(s.G, kNlWarps * 32) : 0;
+        const int links = s.pend_links ? s.G : 0;
         s.pend_links = false;
-        const bool wide = (size_t)s.nb_cap * s.nb_stride > 0xffffffffull;  // list index beyond 32 bits
-        if (half && s.half_ghost)
-            launch_build_list<2>(s, wide, nb + lb, s.rref, a, nb, la);
-        else if (half)
-            launch_build_list<1>(s, wide, nb + lb, s.ref.b[s.ac], a, nb, la);
-        else
-            launch_build_list<0>(s, wide, nb + lb, s.ref.b[s.ac], a, nb, la);
+        if (half && s.half_ghost) launch_build_list<2>(s, s.rref, a, la, links);
+        else if (half) launch_build_list<1>(s, s.ref.b[s.ac], a, la, links);
+        else launch_build_list<0>(s, s.ref.b[s.ac], a, la, links);
         launched(K_NLIST);
         prof_end(K_NLIST);
         TMD_CUDA(cudaMemcpyAsync(s.status_host, s.status_dev, sizeof(DevStatus), cudaMemcpyDeviceToHost, s.stream));

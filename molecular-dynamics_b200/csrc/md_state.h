@@ -93,12 +93,13 @@ struct Geometry {
 // Device-side status words written by kernels and read back with one copy.
 struct DevStatus {
     int nghost;         // ghosts produced by the last border pass
-    // zeroed together before a binning (one memset): out_local .. img_over2
+    // zeroed together before a binning (one memset): out_local .. filled
     int out_local;      // locals outside the cell grid at the last binning
     int out_ghost;      // ghosts outside the cell grid
     int nchain;         // ghosts whose two-phase source is a ghost (last distribution)
     int img_over1;      // locals with more than kImg1 direct images
     int img_over2;      // locals with more than kImg2 images in all
+    int filled;         // cells that hold locals
     int max_nb;         // longest neighbour list of the last build (zeroed before each build)
 };
 
@@ -168,6 +169,7 @@ struct State {
     int nblk_border = 0;
     int lists_valid = 0;
     bool lists_half = false;
+    int cells_filled = 0;  // cells that hold locals, at the last binning whose status was read (0: none)
 
     // modes
     int precision = 0;   // 0 FP64, 1 mixed
