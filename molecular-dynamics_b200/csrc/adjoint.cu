@@ -489,6 +489,7 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     dalloc(&gacc, 2 * (size_t)nbs + 2);
     dfree(&red);
     dalloc(&red, 8);
+    flush_thermo(s);  // sums of a forward run waiting in the scratch
     ensure_red_scratch(s, 8 * nb);
     const double sig6 = std::pow(sigma, 6);
     k_adj_init<<<nb, kT, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.ref.b[s.ac], x0_dev, s.frc.b[s.ac], s.frc32,

@@ -376,6 +376,7 @@ void free_all(State& s) {
     dfree(&s.status_dev);
     s.scan_part_cap = 0;
     s.red_part_cap = 0;
+    s.red_q0 = s.red_q1 = 0;
     s.dev_bytes = 0;
 }
 
@@ -1456,6 +1457,7 @@ int md_get_thermo(double* out) {
     State& s = g_state;
     if (!require_alive("md_get_thermo")) return -1;
     flush_all(s);
+    flush_thermo(s);
     TMD_CUDA(cudaMemcpyAsync(out, s.thermo_dev, 4 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     sync_stream(s);
     s.rsq_iters = (long long)out[2];
@@ -1471,6 +1473,7 @@ int md_thermo_request(void) {
     State& s = g_state;
     if (!require_alive("md_thermo_request")) return -1;
     flush_all(s);
+    flush_thermo(s);
     const long long t = s.thermo_tickets++;
     const int k = (int)(t % kThermoSlots);
     if (s.thermo_slot_ticket[k] >= 0) TMD_CUDA(cudaEventSynchronize(s.thermo_ev[k]));  // slot reused

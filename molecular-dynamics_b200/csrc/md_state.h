@@ -230,6 +230,7 @@ struct State {
     // scan scratch, reductions, status
     int* scan_part = nullptr;  int scan_part_cap = 0;
     double* red_part = nullptr; int red_part_cap = 0;
+    int red_nb = 0, red_q0 = 0, red_q1 = 0;  // quantities [red_q0, red_q1) of red_nb blocks wait there for flush_thermo
     double* thermo_dev = nullptr;   // [8]
     DevStatus* status_dev = nullptr;
     DevStatus* status_host = nullptr;  // pinned
@@ -346,7 +347,6 @@ bool force_init_fusable(const State& s, const PendingForce& p);
 // ghosts of the current buffer from their sources after run_force_lj_init: gm 0 carries
 // them over, 1 is the reference two-phase refresh, 2 exact images
 void run_ghost_refresh(State& s, int gm);
-void run_reduce_thermo(State& s, int nblocks, int nq);
 // multi-rank (k_halo.cu): atoms that left the rank box go to their new owners (the caller
 // flushed pending work); the remote part of a border pass (after its emit); the ghosts
 // received from other ranks refreshed from the current positions of their roots
@@ -357,8 +357,8 @@ bool run_halo_sync(State& s);
 void halo_free(State& s);
 // the per-local arrays sized by the local count (border masks and counts, list stride) hold n
 bool ensure_locals(State& s, int n);
-// sums the [q][nblocks] per-block partials of quantities q0..q1-1 into thermo_dev[q]
-void run_reduce_partials(State& s, int nblocks, int q0, int q1);
+// adds up the partial sums still waiting in red_part into thermo_dev (before it is read)
+void flush_thermo(State& s);
 void exclusive_scan(State& s, const int* in, int* out, int n);
 void ensure_scan_scratch(State& s, int n);
 void ensure_red_scratch(State& s, int n);
