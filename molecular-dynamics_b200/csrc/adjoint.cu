@@ -27,6 +27,7 @@
 
 #include "md_common.cuh"
 #include "comm.h"
+#include "launch.cuh"
 #include "md_state.h"
 #include "tinymd_b200.h"
 
@@ -97,8 +98,9 @@ __global__ void __launch_bounds__(kT)
 k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, double4* __restrict__ w_next,
                 double4* __restrict__ ax, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
                 const int* __restrict__ nbr, double* __restrict__ gacc, HvpArgs a) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kT / 32];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blk * blockDim.x + threadIdx.x;
     const int i = t / kLpa, sub = t % kLpa;
     const bool act = i < a.N;
     double ux = 0.0, uy = 0.0, uz = 0.0, Fx = 0.0, Fy = 0.0, Fz = 0.0, gs = 0.0;
@@ -173,15 +175,16 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
     const double se = block_sum(ge, scratch);
     const double ss = block_sum(gs, scratch);
     if (threadIdx.x == 0) {
-        gacc[blockIdx.x] += a.wt * se;
-        gacc[gridDim.x + blockIdx.x] += a.wt * ss;
+        gacc[blk] += a.wt * se;
+        gacc[gridDim.x + blk] += a.wt * ss;
     }
 }
 
 // the root slot of every list entry (a ghost's root local, a local itself)
 __global__ void k_root_list(const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
                             const int* __restrict__ groot, int* __restrict__ nbr, int N, int stride, int nbcap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int n = min(nbn[i], nbcap);
     for (int k = 0; k < n; ++k) {
@@ -200,8 +203,9 @@ k_adj_init(const double4* __restrict__ pos, const int* __restrict__ img, const i
            int mixed, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, double4* __restrict__ ax,
            double4* __restrict__ av, double* __restrict__ part, int N, int stride, int nbcap, double rc2,
            double sigma6, double eps, double inv_sigma, double len0, double len1, double len2, double dt) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[64];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blk * blockDim.x + threadIdx.x;
     double msd = 0.0, dus = 0.0, ue = 0.0, dus_c = 0.0, ue_c = 0.0, np_ = 0.0, np_c = 0.0;
     if (i < N) {
         const double4 p = pos[i];
@@ -245,33 +249,35 @@ k_adj_init(const double4* __restrict__ pos, const int* __restrict__ img, const i
     block_sum_dd(np_, np_c, scratch);
     if (threadIdx.x == 0) {
         const int nb = gridDim.x;
-        part[blockIdx.x] = msd;
-        part[nb + blockIdx.x] = msd_c;
-        part[2 * nb + blockIdx.x] = dus;
-        part[3 * nb + blockIdx.x] = dus_c;
-        part[4 * nb + blockIdx.x] = ue;
-        part[5 * nb + blockIdx.x] = ue_c;
-        part[6 * nb + blockIdx.x] = np_;
-        part[7 * nb + blockIdx.x] = np_c;
+        part[blk] = msd;
+        part[nb + blk] = msd_c;
+        part[2 * nb + blk] = dus;
+        part[3 * nb + blk] = dus_c;
+        part[4 * nb + blk] = ue;
+        part[5 * nb + blk] = ue_c;
+        part[6 * nb + blk] = np_;
+        part[7 * nb + blk] = np_c;
     }
 }
 
 // out[q] = the compensated total of rows (2q, 2q + 1) of part[.][nb]
 __global__ void k_sum_rows_dd(const double* __restrict__ part, double* __restrict__ out, int nb, int nq) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[64];
     for (int q = 0; q < nq; ++q) {
         double s = 0.0, c = 0.0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) dd_add(s, c, part[2 * q * nb + b], part[(2 * q + 1) * nb + b]);
+        for (int b = threadIdx.x + blk; b < nb; b += blockDim.x) dd_add(s, c, part[2 * q * nb + b], part[(2 * q + 1) * nb + b]);
         block_sum_dd(s, c, scratch);
         if (threadIdx.x == 0) out[q] = s + c;
     }
 }
 
 __global__ void k_sum_rows(const double* __restrict__ part, double* __restrict__ out, int nb, int rows) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[32];
     for (int q = 0; q < rows; ++q) {
         double v = 0.0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) v += part[q * nb + b];
+        for (int b = threadIdx.x + blk; b < nb; b += blockDim.x) v += part[q * nb + b];
         const double r = block_sum(v, scratch);
         if (threadIdx.x == 0) out[q] = r;
     }
@@ -280,20 +286,23 @@ __global__ void k_sum_rows(const double* __restrict__ part, double* __restrict__
 // slot order -> reference order (locals)
 __global__ void k_to_ref(const double4* __restrict__ src, const int* __restrict__ ref, double4* __restrict__ dst,
                          int N) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int s = blk * blockDim.x + threadIdx.x;
     if (s < N) dst[ref[s]] = src[s];
 }
 // reference order -> slot order (locals)
 __global__ void k_from_ref(const double4* __restrict__ src, const int* __restrict__ ref, double4* __restrict__ dst,
                            int N) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int s = blk * blockDim.x + threadIdx.x;
     if (s < N) dst[s] = src[ref[s]];
 }
 // checkpoint of the current state in reference order
 __global__ void k_checkpoint(const double4* __restrict__ pos, const double4* __restrict__ vel,
                              const int* __restrict__ img, const int* __restrict__ ref, double4* __restrict__ cx,
                              double4* __restrict__ cv, int* __restrict__ ci, int N) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int s = blk * blockDim.x + threadIdx.x;
     if (s < N) {
         const int r = ref[s];
         cx[r] = pos[s];
@@ -306,7 +315,8 @@ __global__ void k_restore(const double4* __restrict__ cx, const double4* __restr
                           const int* __restrict__ ci, const double* __restrict__ mass_ref, double4* __restrict__ pos,
                           double4* __restrict__ vel, int* __restrict__ img, int* __restrict__ ref,
                           int* __restrict__ slot_of_ref, double* __restrict__ mass, int N) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int r = blk * blockDim.x + threadIdx.x;
     if (r < N) {
         pos[r] = cx[r];
         vel[r] = cv[r];
@@ -345,9 +355,8 @@ void reset_identity(State& s, int ckpt) {
     const int N = s.N;
     s.G = 0;
     s.pc = s.vc = s.ac = 0;
-    k_restore<<<nblk(N), kT, 0, s.stream>>>(ck_x + (size_t)ckpt * N, ck_v + (size_t)ckpt * N,
-                                           ck_img + (size_t)ckpt * N, mass_ref, s.pos.b[0], s.vel.b[0], s.img.b[0],
-                                           s.ref.b[0], s.slot_of_ref, s.mass.b[0], N);
+    launch(s, nblk(N), kT, 0, k_restore, ck_x + (size_t)ckpt * N, ck_v + (size_t)ckpt * N, ck_img + (size_t)ckpt * N,
+           mass_ref, s.pos.b[0], s.vel.b[0], s.img.b[0], s.ref.b[0], s.slot_of_ref, s.mass.b[0], N);
     launched(K_ADJ_STEP);
 }
 
@@ -362,8 +371,8 @@ PendingForce force_params() {
 
 void checkpoint(State& s, int k) {
     const int N = s.N;
-    k_checkpoint<<<nblk(N), kT, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc], s.img.b[s.ac], s.ref.b[s.ac],
-                                              ck_x + (size_t)k * N, ck_v + (size_t)k * N, ck_img + (size_t)k * N, N);
+    launch(s, nblk(N), kT, 0, k_checkpoint, s.pos.b[s.pc], s.vel.b[s.vc], s.img.b[s.ac], s.ref.b[s.ac],
+           ck_x + (size_t)k * N, ck_v + (size_t)k * N, ck_img + (size_t)k * N, N);
     launched(K_ADJ_STEP);
 }
 
@@ -492,12 +501,11 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     flush_thermo(s);  // sums of a forward run waiting in the scratch
     ensure_red_scratch(s, 8 * nb);
     const double sig6 = std::pow(sigma, 6);
-    k_adj_init<<<nb, kT, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.ref.b[s.ac], x0_dev, s.frc.b[s.ac], s.frc32,
-                                       s.precision, s.nbn, s.nbl, ax, av[0], s.red_part, N, s.nb_stride, s.nb_cap,
-                                       cfg.cutoff * cfg.cutoff, sig6, epsilon, 1.0 / sigma, s.geo.len[0],
-                                       s.geo.len[1], s.geo.len[2], cfg.dt);
+    launch(s, nb, kT, 0, k_adj_init, s.pos.b[s.pc], s.img.b[s.ac], s.ref.b[s.ac], x0_dev, s.frc.b[s.ac], s.frc32,
+           s.precision, s.nbn, s.nbl, ax, av[0], s.red_part, N, s.nb_stride, s.nb_cap, cfg.cutoff * cfg.cutoff, sig6,
+           epsilon, 1.0 / sigma, s.geo.len[0], s.geo.len[1], s.geo.len[2], cfg.dt);
     launched(K_ADJ_STEP);
-    k_sum_rows_dd<<<1, 256, 0, s.stream>>>(s.red_part, red, nb, 4);
+    launch(s, 1, 256, 0, k_sum_rows_dd, s.red_part, red, nb, 4);
     launched(K_ADJ_STEP);
     double sums[4] = {0, 0, 0, 0};
     TMD_CUDA(cudaMemcpyAsync(sums, red, sizeof(sums), cudaMemcpyDeviceToHost, s.stream));
@@ -525,10 +533,10 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     g0[2 * (size_t)nbs + 1] = dUds / N;
     TMD_CUDA(cudaMemcpyAsync(gacc, g0.data(), sizeof(double) * g0.size(), cudaMemcpyHostToDevice, s.stream));
     // adjoint state to reference order (the backward pass starts in another layout)
-    k_to_ref<<<nb, kT, 0, s.stream>>>(ax, s.ref.b[s.ac], tmp4, N);
+    launch(s, nb, kT, 0, k_to_ref, ax, s.ref.b[s.ac], tmp4, N);
     launched(K_ADJ_STEP);
     TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
-    k_to_ref<<<nb, kT, 0, s.stream>>>(av[0], s.ref.b[s.ac], tmp4, N);
+    launch(s, nb, kT, 0, k_to_ref, av[0], s.ref.b[s.ac], tmp4, N);
     launched(K_ADJ_STEP);
     TMD_CUDA(cudaMemcpyAsync(av[0], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
     TMD_CUDA(cudaStreamSynchronize(s.stream));
@@ -573,7 +581,7 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
             dalloc(&nbr, nl);
             cap_nbr = nl;
         }
-        k_root_list<<<nb, kT, 0, s.stream>>>(s.nbn, s.nbl, s.groot, nbr, N, s.nb_stride, s.nb_cap);
+        launch(s, nb, kT, 0, k_root_list, s.nbn, s.nbl, s.groot, nbr, N, s.nb_stride, s.nb_cap);
         launched(K_ADJ_STEP);
         run_force_lj(s, force_params(), false, 0.0);
         TMD_CUDA(cudaMemcpyAsync(seg_x, s.pos.b[s.pc], sizeof(double4) * NA, cudaMemcpyDeviceToDevice, s.stream));
@@ -584,10 +592,10 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
         }
         // adjoint state into this segment's slot order
         const int* ref = s.ref.b[s.ac];
-        k_from_ref<<<nb, kT, 0, s.stream>>>(ax, ref, tmp4, N);
+        launch(s, nb, kT, 0, k_from_ref, ax, ref, tmp4, N);
         launched(K_ADJ_STEP);
         TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
-        k_from_ref<<<nb, kT, 0, s.stream>>>(av[wcur], ref, tmp4, N);
+        launch(s, nb, kT, 0, k_from_ref, av[wcur], ref, tmp4, N);
         launched(K_ADJ_STEP);
         TMD_CUDA(cudaMemcpyAsync(av[wcur], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
         HvpArgs a;
@@ -604,22 +612,22 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
             a.drift = t > 0 ? cfg.dt : 0.0;
             a.wt = t > 0 ? cfg.dt : c;
             prof_begin(K_HVP);
-            k_adj_hvp_split<<<nbs, kT, 0, s.stream>>>(seg_x + (size_t)(t - t0) * NA, av[wcur], av[1 - wcur], ax,
-                                                      s.nbn, s.nbl, nbr, gacc, a);
+            launch(s, nbs, kT, 0, k_adj_hvp_split, seg_x + (size_t)(t - t0) * NA, av[wcur], av[1 - wcur], ax, s.nbn,
+                   s.nbl, nbr, gacc, a);
             launched(K_HVP);
             prof_end(K_HVP);
             wcur = 1 - wcur;
         }
-        k_to_ref<<<nb, kT, 0, s.stream>>>(ax, ref, tmp4, N);
+        launch(s, nb, kT, 0, k_to_ref, ax, ref, tmp4, N);
         launched(K_ADJ_STEP);
         TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
-        k_to_ref<<<nb, kT, 0, s.stream>>>(av[wcur], ref, tmp4, N);
+        launch(s, nb, kT, 0, k_to_ref, av[wcur], ref, tmp4, N);
         launched(K_ADJ_STEP);
         TMD_CUDA(cudaMemcpyAsync(av[wcur], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
     }
     cudaEventRecord(e1, s.stream);
     // theta gradients: per-block sums plus the direct terms stored after them
-    k_sum_rows<<<1, 256, 0, s.stream>>>(gacc, red, nbs, 2);
+    launch(s, 1, 256, 0, k_sum_rows, gacc, red, nbs, 2);
     launched(K_ADJ_STEP);
     double gsum[2] = {0, 0}, direct[2] = {0, 0};
     std::vector<double4> hv(N);

@@ -20,6 +20,7 @@
 
 #include "comm.h"
 #include "md_common.cuh"
+#include "launch.cuh"
 #include "md_state.h"
 #include "tinymd_b200.h"
 
@@ -594,7 +595,8 @@ __global__ void k_gather_ref(const double4* __restrict__ pos, const double4* __r
                              const double4* __restrict__ frc, const float4* __restrict__ frc32,
                              const double* __restrict__ mass, const int* __restrict__ ref, double* __restrict__ out,
                              int N, int NA, int mixed, int ghost_vel) {
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int slot = blk * blockDim.x + threadIdx.x;
     if (slot >= NA) return;
     const int r = ref[slot];
     if (r < 0 || r >= NA) return;
@@ -633,7 +635,8 @@ __global__ void k_upload(const double* __restrict__ m, const double* __restrict_
                          double4* __restrict__ pos, double4* __restrict__ vel, double4* __restrict__ frc,
                          float4* __restrict__ frc32, double* __restrict__ mass, int* __restrict__ ref,
                          int* __restrict__ slot_of_ref, int* __restrict__ img, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const size_t k = 3 * (size_t)i;
     pos[i] = make_double4(p[k], p[k + 1], p[k + 2], 0.0);
@@ -647,7 +650,8 @@ __global__ void k_upload(const double* __restrict__ m, const double* __restrict_
 }
 
 __global__ void k_convert_forces(double4* f64, float4* f32, int n, int to32) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    int i = blk * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (to32) {
         double4 f = f64[i];
@@ -916,8 +920,8 @@ void md_copy_data_to_accelerator(void) {
     TMD_CUDA(cudaMemcpyAsync(dm, s.h_mass.data(), sizeof(double) * N, cudaMemcpyHostToDevice, s.stream));
     TMD_CUDA(cudaMemcpyAsync(dp, s.h_pos.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice, s.stream));
     TMD_CUDA(cudaMemcpyAsync(dv, s.h_vel.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice, s.stream));
-    k_upload<<<(N + 255) / 256, 256, 0, s.stream>>>(dm, dp, dv, s.pos.b[0], s.vel.b[0], s.frc.b[0], s.frc32,
-                                                    s.mass.b[0], s.ref.b[0], s.slot_of_ref, s.img.b[0], N);
+    launch(s, (N + 255) / 256, 256, 0, k_upload, dm, dp, dv, s.pos.b[0], s.vel.b[0], s.frc.b[0], s.frc32,
+           s.mass.b[0], s.ref.b[0], s.slot_of_ref, s.img.b[0], N);
     launched(K_MISC);
     // the mirror may be resized (and moved) by later calls: wait for the copies out of it
     sync_stream(s);
@@ -940,9 +944,8 @@ void md_copy_data_from_accelerator(void) {
     s.h_frc.resize((size_t)NA * 3);
     s.mirror_pending = 0;
     if (NA == 0) return;
-    k_gather_ref<<<(NA + 255) / 256, 256, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac], s.frc32,
-                                                         s.mass.b[s.ac], s.ref.b[s.ac], s.dl_buf, s.N, NA,
-                                                         s.precision == 1, s.dem_fixed);
+    launch(s, (NA + 255) / 256, 256, 0, k_gather_ref, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac], s.frc32,
+           s.mass.b[s.ac], s.ref.b[s.ac], s.dl_buf, s.N, NA, s.precision == 1, s.dem_fixed);
     launched(K_MISC);
     s.mirror_pending = (s.N > 0 ? 1 : 0) | (s.G > 0 ? 2 : 0);
     s.mirror_n = s.N;
@@ -1427,7 +1430,7 @@ void md_set_precision(int mode) {
         flush_all(s);
         const int NA = s.N + s.G;
         if (NA > 0) {
-            k_convert_forces<<<(NA + 255) / 256, 256, 0, s.stream>>>(s.frc.b[s.ac], s.frc32, NA, mode);
+            launch(s, (NA + 255) / 256, 256, 0, k_convert_forces, s.frc.b[s.ac], s.frc32, NA, mode);
             launched(K_MISC);
         }
         s.precision = mode;

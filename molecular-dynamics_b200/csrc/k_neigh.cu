@@ -26,6 +26,7 @@
 
 #include "comm.h"
 #include "md_common.cuh"
+#include "launch.cuh"
 #include "md_state.h"
 
 namespace tmd {
@@ -104,7 +105,8 @@ __device__ __forceinline__ double4 wrap_local(double4* __restrict__ pos, int* __
 }
 
 __global__ void k_enforce_pbc(double4* __restrict__ pos, int* __restrict__ img, int N, GeoArgs a) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    int i = blk * blockDim.x + threadIdx.x;
     if (i >= N) return;
     wrap_local(pos, img, i, a);
 }
@@ -148,8 +150,9 @@ template <bool WRAP>
 __global__ void __launch_bounds__(kBorderThreads) k_border_count(double4* __restrict__ pos, int* __restrict__ img, const int* __restrict__ slot_of_ref,
                                unsigned* __restrict__ bmask, int* __restrict__ bcount, int N, int nblk, GeoArgs a,
                                int* __restrict__ cnt, int nseg, DevStatus* st) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int wc[kBorderThreads / 32][26];
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blk * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // the binning that follows starts from zeroed cell counters and status (no memsets there)
     for (int g = r; g < nseg; g += gridDim.x * blockDim.x) cnt[g] = 0;
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_count(double4* __rest
     if (threadIdx.x < 26) {
         int s = 0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += wc[w][threadIdx.x];
-        bcount[threadIdx.x * nblk + blockIdx.x] = s;
+        bcount[threadIdx.x * nblk + blk] = s;
     }
 }
 
@@ -191,9 +194,10 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
                               int* __restrict__ gsrc, int* __restrict__ groot, int* __restrict__ gcode,
                               int* __restrict__ bsrc_ref, int* __restrict__ broot_ref, int* __restrict__ bcode,
                               int N, int nblk, int capA, GeoArgs a, int sync_vel, RemoteOut ro) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int wpre[kBorderThreads / 32][26];
     __shared__ unsigned char s_rank[26][kBorderThreads];  // a thread's rank among its warp's ghosts of each type
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blk * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned m = r < N ? bmask[r] : 0u;
     const unsigned lt = lanemask_lt();
@@ -219,7 +223,7 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
     const double4 vroot = vel[s_root];
     const unsigned flags = m >> 26;
     // index of this root's ghost of type t (a type whose bit is set)
-    auto gidx = [&](int t) { return boff[t * nblk + blockIdx.x] + wpre[wid][t] + s_rank[t][threadIdx.x]; };
+    auto gidx = [&](int t) { return boff[t * nblk + blk] + wpre[wid][t] + s_rank[t][threadIdx.x]; };
     for (int t = 0; t < 26; ++t) {
         if (!((m >> t) & 1u)) continue;
         if (MR && !((ro.selfmask >> t) & 1u)) {
@@ -277,7 +281,8 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
 // the grid), [ncells+1, 2*ncells+1] ghosts per cell.
 __global__ void k_bin_count(const double4* __restrict__ pos, int* __restrict__ cnt, int* __restrict__ bin_cell,
                             int* __restrict__ bin_rank, DevStatus* st, int N, int NA, GeoArgs a) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    int s = blk * blockDim.x + threadIdx.x;
     if (s >= NA) return;
     int c = flat_cell(pos[s], a);
     if (c == a.ncells) atomicAdd(s < N ? &st->out_local : &st->out_ghost, 1);
@@ -289,7 +294,8 @@ __global__ void k_bin_count(const double4* __restrict__ pos, int* __restrict__ c
 __global__ void k_bin_scatter(const int* __restrict__ ref, const int* __restrict__ bin_cell,
                               const int* __restrict__ bin_rank, const int* __restrict__ cstart,
                               int* __restrict__ tmp_key, int* __restrict__ tmp_src, int N, int NA, int ncells) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    int s = blk * blockDim.x + threadIdx.x;
     if (s >= NA) return;
     int c = bin_cell[s];
     int seg = s < N ? c : (ncells + 1) + c;
@@ -345,7 +351,8 @@ __device__ __forceinline__ void move_slot(int n, int o, const MoveArgs& m, const
 __global__ void k_rank_move(const int* __restrict__ cstart, const int* __restrict__ tmp_key,
                             const int* __restrict__ tmp_src, int NA, int ncells, MoveArgs m, GeoArgs ga,
                             DevStatus* st) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int e = blk * blockDim.x + threadIdx.x;
     // the list build that follows starts from a zeroed status (no memset there)
     if (e == 0) st->max_nb = 0;
     const int o = e < NA ? tmp_src[e] : 0;
@@ -410,7 +417,8 @@ __device__ __forceinline__ void ghost_link(int h, const LinkArgs& l) {
 }
 
 __global__ void k_ghost_links(LinkArgs l) {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int h = blk * blockDim.x + threadIdx.x;
     if (h < l.G) ghost_link(h, l);
 }
 
@@ -538,6 +546,7 @@ __global__ void __launch_bounds__(kNlThreads, 8)
 k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const int* __restrict__ rbk,
              const int* __restrict__ cstart, int* __restrict__ nbn, uint32_t* __restrict__ nbl, DevStatus* st,
              NlArgs a, int cell_blocks, LinkArgs la) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     // candidate position (cell-centre relative); w = slot << 6 + its rebasing cell relative to the
     // first home's (rel_code) + kCodeBias, from which a home's entry is one subtraction
     __shared__ float4 s_cand[kNlTile + 32 * kNlStep];
@@ -555,13 +564,13 @@ k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const
     __shared__ int s_kept[kNlWarps];
     __shared__ __align__(16) uint32_t s_buf[kNlThreads / 32][kNlBuf];
 
-    if ((int)blockIdx.x >= cell_blocks) {  // blocks past the cells link the ghosts (k_ghost_links' work)
-        const int h = (blockIdx.x - cell_blocks) * blockDim.x + threadIdx.x;
+    if (blk >= cell_blocks) {  // blocks past the cells link the ghosts (k_ghost_links' work)
+        const int h = (blk - cell_blocks) * blockDim.x + threadIdx.x;
         if (h < la.G) ghost_link(h, la);
         return;
     }
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x;
+    const int c = blk;
     const int h0 = cstart[c], h1 = cstart[c + 1];
     if (h0 == h1) return;
     const unsigned lt = lanemask_lt();
@@ -829,15 +838,16 @@ __global__ void __launch_bounds__(kSparseThreads)
 k_build_list_sparse(const double4* __restrict__ pos, const int* __restrict__ ref, const int* __restrict__ rbk,
                     const int* __restrict__ cstart, const int* __restrict__ slot_cell, int* __restrict__ nbn,
                     uint32_t* __restrict__ nbl, DevStatus* st, NlArgs a, int local_blocks, LinkArgs la) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     // a home's ranges: candidates before it, first slot minus that
     __shared__ int2 s_range[kSparseThreads / kSparseLanes][55];
-    if ((int)blockIdx.x >= local_blocks) {  // blocks past the locals link the ghosts (k_ghost_links' work)
-        const int h = (blockIdx.x - local_blocks) * blockDim.x + threadIdx.x;
+    if (blk >= local_blocks) {  // blocks past the locals link the ghosts (k_ghost_links' work)
+        const int h = (blk - local_blocks) * blockDim.x + threadIdx.x;
         if (h < la.G) ghost_link(h, la);
         return;
     }
     const int lane = threadIdx.x & 31, l = lane % kSparseLanes;
-    const int i = (blockIdx.x * kSparseThreads + threadIdx.x) / kSparseLanes;
+    const int i = (blk * kSparseThreads + threadIdx.x) / kSparseLanes;
     const unsigned group = 0xffu << (lane - l), before = lanemask_lt() & group;
     int cnt = 0;
     // a home outside the grid (or past the last one) has no candidates; the warp's homes keep together,
@@ -946,7 +956,8 @@ k_build_list_sparse(const double4* __restrict__ pos, const int* __restrict__ ref
 
 // Locals outside the grid (bucket ncells) get empty lists.
 __global__ void k_clear_lists(int* __restrict__ nbn, int a, int b) {
-    int i = a + blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    int i = a + blk * blockDim.x + threadIdx.x;
     if (i < b) nbn[i] = 0;
 }
 
@@ -982,21 +993,23 @@ constexpr int kScanThreads = 1024, kScanItems = 4, kScanBlock = kScanThreads * k
 
 // per-block totals of the input
 __global__ void k_scan_sums(const int* __restrict__ in, int* __restrict__ part, int n) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int sh[32];
-    int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+    int base = blk * kScanBlock + threadIdx.x * kScanItems;
     int s = 0;
     for (int k = 0; k < kScanItems; ++k) s += (base + k < n) ? in[base + k] : 0;
     int tot;
     block_exscan(s, &tot, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = tot;
+    if (threadIdx.x == 0) part[blk] = tot;
 }
 
 // exclusive scan of the block totals in place (one block); part[nb] = grand total
 __global__ void k_scan_part(int* __restrict__ part, int nb) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int sh[32];
     int carry = 0;
     for (int b0 = 0; b0 < nb; b0 += kScanThreads) {
-        int i = b0 + threadIdx.x;
+        int i = b0 + threadIdx.x + blk;
         int v = i < nb ? part[i] : 0;
         int tot;
         int ex = block_exscan(v, &tot, sh);
@@ -1009,8 +1022,9 @@ __global__ void k_scan_part(int* __restrict__ part, int nb) {
 
 __global__ void k_scan_apply(const int* __restrict__ in, int* __restrict__ out, const int* __restrict__ part,
                              int n, int nb) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int sh[32];
-    int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+    int base = blk * kScanBlock + threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
     for (int k = 0; k < kScanItems; ++k) {
@@ -1018,12 +1032,12 @@ __global__ void k_scan_apply(const int* __restrict__ in, int* __restrict__ out, 
         s += v[k];
     }
     int tot;
-    int ex = block_exscan(s, &tot, sh) + part[blockIdx.x];
+    int ex = block_exscan(s, &tot, sh) + part[blk];
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < n) out[base + k] = ex;
         ex += v[k];
     }
-    if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[n] = part[nb];
+    if (blk == nb - 1 && threadIdx.x == 0) out[n] = part[nb];
 }
 
 // Exclusive scan of up to kScanSingleMax values in one block: the values are staged in
@@ -1033,10 +1047,11 @@ __global__ void k_scan_apply(const int* __restrict__ in, int* __restrict__ out, 
 constexpr int kScanSingleMax = 32768;  // 128 KiB of shared memory
 __global__ void __launch_bounds__(kScanThreads) k_scan_single(const int* __restrict__ in, int* __restrict__ out,
                                                                int n) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     extern __shared__ int sv[];
     __shared__ int sh[32];
 #pragma unroll 8
-    for (int k = threadIdx.x; k < n; k += kScanThreads) sv[k] = in[k];
+    for (int k = threadIdx.x + blk; k < n; k += kScanThreads) sv[k] = in[k];
     __syncthreads();
     const int run = (n + kScanThreads - 1) / kScanThreads;
     const int base = threadIdx.x * run;
@@ -1075,9 +1090,10 @@ __device__ __forceinline__ unsigned long long lb_word(unsigned epoch, unsigned s
 __global__ void __launch_bounds__(kLbThreads)
 k_scan_lookback(const int* __restrict__ in, int* __restrict__ out, int n, int ntiles,
                 unsigned long long* __restrict__ tiles, unsigned epoch) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ int sh[32];
     __shared__ int s_prefix, s_missing;
-    const int tile = blockIdx.x;
+    const int tile = blk;
     const int base = tile * kLbTile + threadIdx.x * kLbItems;
     int v[kLbItems];
     int sum = 0;
@@ -1171,7 +1187,7 @@ void exclusive_scan(State& s, const int* in, int* out, int n) {
     if (n >= kLookbackMin) {
         const int ntiles = nblocks(n, kLbTile);
         if (ensure_lookback(s, ntiles)) {
-            k_scan_lookback<<<ntiles, kLbThreads, 0, s.stream>>>(in, out, n, ntiles, s.lb_tiles, ++s.lb_epoch);
+            launch(s, ntiles, kLbThreads, 0, k_scan_lookback, in, out, n, ntiles, s.lb_tiles, ++s.lb_epoch);
             launched(K_SCAN);
             return;
         }
@@ -1182,18 +1198,18 @@ void exclusive_scan(State& s, const int* in, int* out, int n) {
                                           kScanSingleMax * (int)sizeof(int)));
             s.scan_attr_device = s.device;
         }
-        k_scan_single<<<1, kScanThreads, (size_t)n * sizeof(int), s.stream>>>(in, out, n);
+        launch(s, 1, kScanThreads, (size_t)n * sizeof(int), k_scan_single, in, out, n);
         launched(K_SCAN);
         return;
     }
     int nb = nblocks(n, kScanBlock);
     if (nb < 1) nb = 1;
     ensure_scan_scratch(s, n);
-    k_scan_sums<<<nb, kScanThreads, 0, s.stream>>>(in, s.scan_part, n);
+    launch(s, nb, kScanThreads, 0, k_scan_sums, in, s.scan_part, n);
     launched(K_SCAN);
-    k_scan_part<<<1, kScanThreads, 0, s.stream>>>(s.scan_part, nb);
+    launch(s, 1, kScanThreads, 0, k_scan_part, s.scan_part, nb);
     launched(K_SCAN);
-    k_scan_apply<<<nb, kScanThreads, 0, s.stream>>>(in, out, s.scan_part, n, nb);
+    launch(s, nb, kScanThreads, 0, k_scan_apply, in, out, s.scan_part, n, nb);
     launched(K_SCAN);
 }
 
@@ -1201,7 +1217,7 @@ void run_enforce_pbc(State& s) {
     if (s.N == 0) return;
     GeoArgs a = geo_args(s.geo);
     prof_begin(K_PBC);
-    k_enforce_pbc<<<nblocks(s.N, 256), 256, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.N, a);
+    launch(s, nblocks(s.N, 256), 256, 0, k_enforce_pbc, s.pos.b[s.pc], s.img.b[s.ac], s.N, a);
     launched(K_PBC);
     prof_end(K_PBC);
 }
@@ -1227,13 +1243,11 @@ void run_borders(State& s, bool wrap) {
         // a rank without locals still takes part in the exchange
         if (N > 0) {
             if (wrap)
-                k_border_count<true><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref,
-                                                                  s.bmask, s.bcount, N, nblk, a, s.cnt, nseg,
-                                                                  s.status_dev);
+                launch(s, nblk, kBorderThreads, 0, k_border_count<true>, s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref,
+                       s.bmask, s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
             else
-                k_border_count<false><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref,
-                                                                   s.bmask, s.bcount, N, nblk, a, s.cnt, nseg,
-                                                                   s.status_dev);
+                launch(s, nblk, kBorderThreads, 0, k_border_count<false>, s.pos.b[s.pc], s.img.b[s.ac],
+                       s.slot_of_ref, s.bmask, s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
             s.bin_zeroed = true;
             launched(K_BORDER);
             exclusive_scan(s, s.bcount, boff, n);
@@ -1242,10 +1256,9 @@ void run_borders(State& s, bool wrap) {
         if (ok && N + s.halo.gself > s.capA) ok = grow_atoms(s, N + s.halo.gself);
         if (ok && N > 0) {
             RemoteOut ro{s.halo.tab, s.halo.send_ref, s.halo.send_type, comm().topo.selfmask};
-            k_border_emit<true><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
-                                                             s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff,
-                                                             s.gsrc, s.groot, s.gcode, s.bsrc_ref, s.broot_ref,
-                                                             s.bcode, N, nblk, s.capA, a, s.dem_fixed, ro);
+            launch(s, nblk, kBorderThreads, 0, k_border_emit<true>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
+                   s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot, s.gcode, s.bsrc_ref,
+                   s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, ro);
             launched(K_BORDER);
         }
         if (ok) ok = halo_finish_borders(s);
@@ -1255,11 +1268,11 @@ void run_borders(State& s, bool wrap) {
         return;
     }
     if (wrap)
-        k_border_count<true><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref, s.bmask,
-                                                          s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
+        launch(s, nblk, kBorderThreads, 0, k_border_count<true>, s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref,
+               s.bmask, s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
     else
-        k_border_count<false><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref, s.bmask,
-                                                           s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
+        launch(s, nblk, kBorderThreads, 0, k_border_count<false>, s.pos.b[s.pc], s.img.b[s.ac], s.slot_of_ref,
+               s.bmask, s.bcount, N, nblk, a, s.cnt, nseg, s.status_dev);
     s.bin_zeroed = true;
     launched(K_BORDER);
     exclusive_scan(s, s.bcount, boff, n);
@@ -1274,10 +1287,9 @@ void run_borders(State& s, bool wrap) {
     TMD_CUDA(cudaMemcpyAsync(&s.status_host->nghost, boff + n, sizeof(int), cudaMemcpyDeviceToHost, s.copy_stream));
     TMD_CUDA(cudaEventRecord(s.ev_counted, s.copy_stream));
     auto emit = [&]() {
-        k_border_emit<false><<<nblk, kBorderThreads, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac], s.mass.b[s.ac],
-                                                  s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot,
-                                                  s.gcode, s.bsrc_ref, s.broot_ref, s.bcode, N, nblk, s.capA,
-                                                  a, s.dem_fixed, RemoteOut{nullptr, nullptr, nullptr, 0u});
+        launch(s, nblk, kBorderThreads, 0, k_border_emit<false>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
+               s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot, s.gcode, s.bsrc_ref,
+               s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, RemoteOut{nullptr, nullptr, nullptr, 0u});
         launched(K_BORDER);
     };
     emit();
@@ -1308,12 +1320,12 @@ void run_distribute(State& s) {
         TMD_CUDA(cudaMemsetAsync(&s.status_dev->out_local, 0, 6 * sizeof(int), s.stream));  // .. filled
     }
     s.bin_zeroed = false;
-    k_bin_count<<<nblocks(NA, 256), 256, 0, s.stream>>>(s.pos.b[s.pc], s.cnt, s.bin_cell, s.bin_rank, s.status_dev,
-                                                        N, NA, a);
+    launch(s, nblocks(NA, 256), 256, 0, k_bin_count, s.pos.b[s.pc], s.cnt, s.bin_cell, s.bin_rank, s.status_dev, N,
+           NA, a);
     launched(K_BIN);
     exclusive_scan(s, s.cnt, s.cstart, nseg);
-    k_bin_scatter<<<nblocks(NA, 256), 256, 0, s.stream>>>(s.ref.b[s.ac], s.bin_cell, s.bin_rank, s.cstart,
-                                                          s.tmp_key, s.tmp_src, N, NA, a.ncells);
+    launch(s, nblocks(NA, 256), 256, 0, k_bin_scatter, s.ref.b[s.ac], s.bin_cell, s.bin_rank, s.cstart, s.tmp_key,
+           s.tmp_src, N, NA, a.ncells);
     launched(K_BIN);
     const int np = 1 - s.pc, nv = 1 - s.vc, na = 1 - s.ac;
     MoveArgs m;
@@ -1327,8 +1339,8 @@ void run_distribute(State& s) {
     m.bin_cell = s.bin_cell; m.slot_cell = s.slot_cell;
     m.pos32 = s.pos32.b[np]; m.img_cnt = s.img_cnt; m.img_slot = s.img_slot;
     m.capA = s.capA; m.N = N; m.mixed = s.precision;
-    k_rank_move<<<nblocks(NA, 256), 256, 0, s.stream>>>(s.cstart, s.tmp_key, s.tmp_src, NA, a.ncells, m, a,
-                                                         s.status_dev);
+    launch(s, nblocks(NA, 256), 256, 0, k_rank_move, s.cstart, s.tmp_key, s.tmp_src, NA, a.ncells, m, a,
+           s.status_dev);
     launched(K_BIN);
     s.build_zeroed = true;
     s.pc = np;
@@ -1369,7 +1381,7 @@ LinkArgs link_args(State& s) {
 void flush_links(State& s) {
     if (!s.pend_links) return;
     s.pend_links = false;
-    k_ghost_links<<<nblocks(s.G, 256), 256, 0, s.stream>>>(link_args(s));
+    launch(s, nblocks(s.G, 256), 256, 0, k_ghost_links, link_args(s));
     launched(K_BIN);
 }
 
@@ -1391,11 +1403,11 @@ void launch_build_list(State& s, const int* ref, const NlArgs& a, const LinkArgs
     const int lb = nblocks(links, kNlThreads);
     if (sparse_cells(s)) {
         const int nb = nblocks((long long)s.N * kSparseLanes, kSparseThreads);
-        k_build_list_sparse<HM><<<nb + lb, kSparseThreads, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart, s.slot_cell,
-                                                                          s.nbn, s.nbl, s.status_dev, a, nb, la);
+        launch(s, nb + lb, kSparseThreads, 0, k_build_list_sparse<HM>, s.pos.b[s.pc], ref, s.rbk, s.cstart,
+               s.slot_cell, s.nbn, s.nbl, s.status_dev, a, nb, la);
     } else {
-        k_build_list<HM><<<a.ncells + lb, kNlThreads, 0, s.stream>>>(s.pos.b[s.pc], ref, s.rbk, s.cstart, s.nbn, s.nbl,
-                                                                     s.status_dev, a, a.ncells, la);
+        launch(s, a.ncells + lb, kNlThreads, 0, k_build_list<HM>, s.pos.b[s.pc], ref, s.rbk, s.cstart, s.nbn, s.nbl,
+               s.status_dev, a, a.ncells, la);
     }
 }
 
@@ -1409,7 +1421,7 @@ static int finish_build(State& s, bool half) {
         // locals outside the grid sit at [cstart[ncells], N): empty lists
         TMD_CUDA(cudaMemcpyAsync(&first_out, s.cstart + g.ncells, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
         TMD_CUDA(cudaStreamSynchronize(s.stream));
-        k_clear_lists<<<nblocks(s.N - first_out, 256), 256, 0, s.stream>>>(s.nbn, first_out, s.N);
+        launch(s, nblocks(s.N - first_out, 256), 256, 0, k_clear_lists, s.nbn, first_out, s.N);
         launched(K_NLIST);
         set_error(5, "locals outside the cell grid at binning (they have no neighbours)");
     }

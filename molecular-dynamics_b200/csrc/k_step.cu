@@ -13,6 +13,7 @@
 // warp one coalesced 128-byte line per neighbour slot, and neighbour
 // positions come through the read-only path.
 
+#include "launch.cuh"
 #include "lj_args.cuh"
 #include "md_common.cuh"
 #include "md_state.h"
@@ -183,9 +184,10 @@ __global__ void __launch_bounds__(kThreads)
 k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
           const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot,
           double* __restrict__ part, LjArgs a, double4* __restrict__ pos_n = nullptr, PushArgs pa = PushArgs()) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kThreads / 32];
     if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blk * blockDim.x + threadIdx.x;
     const int n = i < a.N ? min(nbn[i], a.nbcap) : 0;
     prefetch_share(pos, (size_t)a.NA * sizeof(double4));
     if (FUSE) prefetch_share(vel, (size_t)a.N * sizeof(double4));
@@ -367,9 +369,10 @@ __global__ void __launch_bounds__(kThreads, TMD_MINB)
 k_lj_mixed_half(const float4* __restrict__ pos32, const double4* __restrict__ pos, float4* __restrict__ frc32,
                 const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot,
                 double* __restrict__ part, LjArgs a) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kThreads / 32];
     __shared__ int s_q[kQQ + 1][kThreads];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blk * blockDim.x + threadIdx.x;
     const int n = i < a.N ? min(nbn[i], a.nbcap) : 0;
     prefetch_share(pos32, (size_t)a.NA * sizeof(float4));
     prefetch_share(pos, (size_t)a.N * sizeof(double4));
@@ -508,12 +511,13 @@ k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos,
               double* __restrict__ part, LjArgs a, double4* __restrict__ pos_n = nullptr,
               float4* __restrict__ pos32_n = nullptr, const int* __restrict__ rbk = nullptr,
               PushArgs pa = PushArgs()) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kThreads / 32];
     // each thread's queue of list quads holding FP64-path pairs: quad index << kB32 | pair bits;
     // row kQQ takes the writes past a full queue
     __shared__ int s_q[kQQ + 1][kThreads];
     if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blk * blockDim.x + threadIdx.x;
     const int n = i < a.N ? min(nbn[i], a.nbcap) : 0;
     prefetch_share(pos32, (size_t)a.NA * sizeof(float4));
     prefetch_share(pos, (size_t)a.N * sizeof(double4));
@@ -653,12 +657,13 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
                  double* __restrict__ part, LjArgs a, int atom_blocks, double4* __restrict__ pos_n = nullptr,
                  float4* __restrict__ pos32_n = nullptr, const int* __restrict__ rbk = nullptr,
                  PushArgs pa = PushArgs()) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kThreads / 32];
     __shared__ int s_q[kQQ + 1][kThreads];
     if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
     double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
-    if ((int)blockIdx.x < atom_blocks) {
-        const int t = blockIdx.x * kThreads + threadIdx.x;
+    if (blk < atom_blocks) {
+        const int t = blk * kThreads + threadIdx.x;
         const int i = t / L, sub = t % L;
         const bool act = i < a.N;
         const int n = act ? min(nbn[i], a.nbcap) : 0;
@@ -742,7 +747,7 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
             cnt = (double)ncnt;
         }
     } else if (PUSH) {
-        push_chain_block<true>((int)blockIdx.x - atom_blocks, pos, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
+        push_chain_block<true>(blk - atom_blocks, pos, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
     }
     if (THERMO) {
         put_partial(part, 0, e, scratch);
@@ -762,6 +767,7 @@ __global__ void __launch_bounds__(kThreads)
 k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
                 const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, double* __restrict__ part, LjArgs a,
                 int atom_blocks, double4* __restrict__ pos_n = nullptr, PushArgs pa = PushArgs()) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     static_assert(L >= 4 && L <= 32, "three lanes of an atom add its force's components");
     // pairs outside the cutoff evaluated too, without a branch: shorter chains (2,048 atoms, 8 lanes:
     // step 12.9 -> 12.2 us) but more work (16,384 atoms, 4 lanes: 18.1 -> 19.2 us)
@@ -775,9 +781,9 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
     __shared__ __align__(16) double s_p[kThreads / 32][kAtoms * kAtom];
     if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
     double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
-    if ((int)blockIdx.x < atom_blocks) {
+    if (blk < atom_blocks) {
         const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int t = blockIdx.x * kThreads + threadIdx.x;
+        const int t = blk * kThreads + threadIdx.x;
         const int i = t / L, sub = t % L, at = lane / L;
         const bool act = i < a.N;
         const int n = act ? min(nbn[i], a.nbcap) : 0;
@@ -853,7 +859,7 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
             if (act && sub == 0) vel[i] = v;
         }
     } else if (PUSH) {
-        push_chain_block<false>((int)blockIdx.x - atom_blocks, pos, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
+        push_chain_block<false>(blk - atom_blocks, pos, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
     }
     if (THERMO) {
         put_partial(part, 0, e, scratch);
@@ -912,7 +918,8 @@ template <bool HALF>
 __global__ void __launch_bounds__(kThreads)
 k_dem_fp64(const double4* __restrict__ pos, const double4* __restrict__ vel, double4* __restrict__ frc,
            const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot, DemArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
     if (i >= a.N) return;
     const double4 pi = pos[i];
     const double4 vi = vel[i];
@@ -966,7 +973,8 @@ __global__ void __launch_bounds__(kThreads)
 k_dem_mixed(const float4* __restrict__ pos32, const double4* __restrict__ pos, const double4* __restrict__ vel,
             float4* __restrict__ frc32, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
             const int* __restrict__ groot, DemArgs a, DemMixedArgs b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
     if (i >= a.N) return;
     float fx = 0.f, fy = 0.f, fz = 0.f;
     double cx = 0.0, cy = 0.0, cz = 0.0;
@@ -1078,7 +1086,8 @@ k_integrate(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, cons
             double4* __restrict__ vel_n, const double4* __restrict__ frc, const float4* __restrict__ frc32,
             const float4* __restrict__ pos32_o, float4* __restrict__ pos32_n, const int* __restrict__ rbk,
             const int* __restrict__ gsrc, const int* __restrict__ groot, const int* __restrict__ gcode, StepArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int t = blk * blockDim.x + threadIdx.x;
     if (t < a.N) {
         double4 v = vel_o[t];
         double fx, fy, fz;
@@ -1137,7 +1146,8 @@ k_ghost_sync(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, con
              float4* __restrict__ pos32_n, double4* __restrict__ vel, int demv, const int* __restrict__ rbk,
              const int* __restrict__ gsrc, const int* __restrict__ groot, const int* __restrict__ gcode,
              StepArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int t = blk * blockDim.x + threadIdx.x;
     if (t < a.N) {
         pos_n[t] = pos_o[t];
         if (MIXED) pos32_n[t] = pos32_o[t];
@@ -1169,7 +1179,8 @@ __global__ void __launch_bounds__(kThreads)
 k_ghost_refresh(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, const float4* __restrict__ pos32_o,
                 float4* __restrict__ pos32_n, const int* __restrict__ rbk, const int* __restrict__ gsrc,
                 const int* __restrict__ groot, const int* __restrict__ gcode, StepArgs a) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int g = blk * blockDim.x + threadIdx.x;
     if (g >= a.G) return;
     const int t = a.N + g;
     if (GM == 0) {
@@ -1195,8 +1206,9 @@ template <bool MIXED, bool THERMO>
 __global__ void __launch_bounds__(kThreads)
 k_final(double4* __restrict__ vel, const double4* __restrict__ frc, const float4* __restrict__ frc32,
         double* __restrict__ part, int N, double h) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[kThreads / 32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blk * blockDim.x + threadIdx.x;
     double ke = 0.0;
     if (i < N) {
         double fx, fy, fz;
@@ -1217,7 +1229,8 @@ k_final(double4* __restrict__ vel, const double4* __restrict__ frc, const float4
 __global__ void k_count_inside(const double4* __restrict__ pos, const int* __restrict__ nbn,
                                const uint32_t* __restrict__ nbl, int N, int stride, int nbcap, double rc2,
                                unsigned long long* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
     unsigned c = 0;
     if (i < N) {
         const double4 pi = pos[i];
@@ -1233,12 +1246,14 @@ __global__ void k_count_inside(const double4* __restrict__ pos, const int* __res
 
 __global__ void k_refresh_pos32(const double4* __restrict__ pos, float4* __restrict__ pos32,
                                 const int* __restrict__ rbk, int NA, StepArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int t = blk * blockDim.x + threadIdx.x;
     if (t < NA) pos32[t] = rebased32(pos[t], rbk[t], a.alo, a.rb_h);
 }
 
 __global__ void k_zero4(double4* __restrict__ d, float4* __restrict__ f, int n) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int t = blk * blockDim.x + threadIdx.x;
     if (t >= n) return;
     if (d) d[t] = make_double4(0.0, 0.0, 0.0, 0.0);
     if (f) f[t] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1247,10 +1262,11 @@ __global__ void k_zero4(double4* __restrict__ d, float4* __restrict__ f, int n) 
 // sums part[q][0..nb) in a fixed order for q in [q0, q1) into out[q]
 __global__ void k_reduce_partials(const double* __restrict__ part, double* __restrict__ out, int nb, int q0,
                                   int q1) {
+    const int blk = (int)blockIdx.x + pdl_wait();
     __shared__ double scratch[32];
     for (int q = q0; q < q1; ++q) {
         double v = 0.0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) v += part[q * nb + b];
+        for (int b = threadIdx.x + blk; b < nb; b += blockDim.x) v += part[q * nb + b];
         double r = block_sum(v, scratch);
         if (threadIdx.x == 0) out[q] = r;
     }
@@ -1295,18 +1311,17 @@ int force_blocks(int N, int lanes, int nchain) {
 
 template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
 void launch_lj_mixed_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
-    k_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
-        s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a,
-        nblocks((long long)a.N * L, kThreads), INIT ? s.pos.b[1 - s.pc] : nullptr,
-        INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
+    launch(s, nb, kThreads, 0, (k_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos32.b[s.pc], s.pos.b[s.pc],
+           s.frc32, s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a, nblocks((long long)a.N * L, kThreads),
+           INIT ? s.pos.b[1 - s.pc] : nullptr, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
 }
 
 template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
 void launch_lj_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
     if (s.precision == 1) return launch_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
-    k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
-        s.pos.b[s.pc], s.frc.b[s.ac], s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a,
-        nblocks((long long)a.N * L, kThreads), INIT ? s.pos.b[1 - s.pc] : nullptr, pa);
+    launch(s, nb, kThreads, 0, (k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac],
+           s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a, nblocks((long long)a.N * L, kThreads),
+           INIT ? s.pos.b[1 - s.pc] : nullptr, pa);
 }
 
 // INIT: the kernels write the integrated locals into the other position buffer
@@ -1327,15 +1342,14 @@ void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs&
     }
     if (s.precision == 1) {
         if constexpr (HALF)
-            k_lj_mixed_half<THERMO><<<nb, kThreads, 0, s.stream>>>(s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.nbn,
-                                                                   s.nbl, s.groot, s.red_part, a);
+            launch(s, nb, kThreads, 0, k_lj_mixed_half<THERMO>, s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.nbn,
+                   s.nbl, s.groot, s.red_part, a);
         else
-            k_lj_mixed_bf<FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
-                s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, vel, s.nbn, s.nbl, s.red_part, a, pn,
-                INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
+            launch(s, nb, kThreads, 0, (k_lj_mixed_bf<FUSE, THERMO, INIT, PUSH>), s.pos32.b[s.pc], s.pos.b[s.pc],
+                   s.frc32, vel, s.nbn, s.nbl, s.red_part, a, pn, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
     } else
-        k_lj_fp64<HALF, FUSE, THERMO, INIT, PUSH><<<nb, kThreads, 0, s.stream>>>(
-            s.pos.b[s.pc], s.frc.b[s.ac], vel, s.nbn, s.nbl, s.groot, s.red_part, a, pn, pa);
+        launch(s, nb, kThreads, 0, (k_lj_fp64<HALF, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac], vel,
+               s.nbn, s.nbl, s.groot, s.red_part, a, pn, pa);
 }
 
 }  // namespace
@@ -1345,7 +1359,7 @@ void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs&
 // every step took 4-6 us of it, 13 of 42 us a step at 29,716 atoms with the sums read every 10 steps.
 void flush_thermo(State& s) {
     if (s.red_q1 <= s.red_q0) return;
-    k_reduce_partials<<<1, 256, 0, s.stream>>>(s.red_part, s.thermo_dev, s.red_nb, s.red_q0, s.red_q1);
+    launch(s, 1, 256, 0, k_reduce_partials, s.red_part, s.thermo_dev, s.red_nb, s.red_q0, s.red_q1);
     launched(K_REDUCE);
     s.red_q0 = s.red_q1 = 0;
 }
@@ -1406,9 +1420,9 @@ void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt) {
     }
     if (half) {
         if (s.precision == 1)
-            k_zero4<<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(nullptr, s.frc32, N);
+            launch(s, nblocks(N, kThreads), kThreads, 0, k_zero4, nullptr, s.frc32, N);
         else
-            k_zero4<<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(s.frc.b[s.ac], nullptr, N);
+            launch(s, nblocks(N, kThreads), kThreads, 0, k_zero4, s.frc.b[s.ac], nullptr, N);
         launched(K_MISC);
         fuse_final = false;
     }
@@ -1513,8 +1527,8 @@ void run_ghost_refresh(State& s, int gm) {
     float4* p32n = s.pos32.b[s.pc];
     const int nb = nblocks(s.G, kThreads);
     const bool mixed = s.precision == 1;
-#define TMD_GR(GM_, MX_) \
-    k_ghost_refresh<GM_, MX_><<<nb, kThreads, 0, s.stream>>>(po, pn, p32o, p32n, s.rbk, s.gsrc, s.groot, s.gcode, a)
+#define TMD_GR(GM_, MX_)                                                                                      \
+    launch(s, nb, kThreads, 0, (k_ghost_refresh<GM_, MX_>), po, pn, p32o, p32n, s.rbk, s.gsrc, s.groot, s.gcode, a)
     prof_begin(K_GHOST_SYNC);
     if (gm == 0) { if (mixed) TMD_GR(0, true); else TMD_GR(0, false); }
     else if (gm == 1) { if (mixed) TMD_GR(1, true); else TMD_GR(1, false); }
@@ -1555,31 +1569,31 @@ void run_force_dem(State& s, const PendingForce& p) {
         b.hy = (float)(-s.geo.rb_h / 4.0);
         b.hz = (float)(-s.geo.rb_h / 16.0);
         if (p.half) {
-            k_zero4<<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(nullptr, s.frc32, N);
+            launch(s, nblocks(N, kThreads), kThreads, 0, k_zero4, nullptr, s.frc32, N);
             launched(K_MISC);
         }
         prof_begin(K_FORCE_DEM);
         if (p.half)
-            k_dem_mixed<true><<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(
-                s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
+            launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_mixed<true>, s.pos32.b[s.pc], s.pos.b[s.pc],
+                   s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
         else
-            k_dem_mixed<false><<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(
-                s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
+            launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_mixed<false>, s.pos32.b[s.pc], s.pos.b[s.pc],
+                   s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
         launched(K_FORCE_DEM);
         prof_end(K_FORCE_DEM);
         return;
     }
     if (p.half) {
-        k_zero4<<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(s.frc.b[s.ac], nullptr, N);
+        launch(s, nblocks(N, kThreads), kThreads, 0, k_zero4, s.frc.b[s.ac], nullptr, N);
         launched(K_MISC);
     }
     prof_begin(K_FORCE_DEM);
     if (p.half)
-        k_dem_fp64<true><<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc],
-                                                                          s.frc.b[s.ac], s.nbn, s.nbl, s.groot, a);
+        launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_fp64<true>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
+               s.nbn, s.nbl, s.groot, a);
     else
-        k_dem_fp64<false><<<nblocks(N, kThreads), kThreads, 0, s.stream>>>(s.pos.b[s.pc], s.vel.b[s.vc],
-                                                                           s.frc.b[s.ac], s.nbn, s.nbl, s.groot, a);
+        launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_fp64<false>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
+               s.nbn, s.nbl, s.groot, a);
     launched(K_FORCE_DEM);
     prof_end(K_FORCE_DEM);
 }
@@ -1602,9 +1616,9 @@ void run_integrate(State& s, double dt, bool fuse_ghosts, double kick_dt) {
     const float4* p32o = s.pos32.b[s.pc];
     float4* p32n = s.pos32.b[1 - s.pc];
     const int nb = nblocks(NA, kThreads);
-#define TMD_INT(GM_, MX_, DV_)                                                                                 \
-    k_integrate<GM_, MX_, DV_><<<nb, kThreads, 0, s.stream>>>(po, pn, vo, vn, s.frc.b[s.ac], s.frc32, p32o, p32n,  \
-                                                              s.rbk, s.gsrc, s.groot, s.gcode, a)
+#define TMD_INT(GM_, MX_, DV_)                                                                                \
+    launch(s, nb, kThreads, 0, (k_integrate<GM_, MX_, DV_>), po, pn, vo, vn, s.frc.b[s.ac], s.frc32, p32o,     \
+           p32n, s.rbk, s.gsrc, s.groot, s.gcode, a)
     prof_begin(K_INTEGRATE);
     if (gm == 0) {
         if (mixed) { if (demv) TMD_INT(0, true, true); else TMD_INT(0, true, false); }
@@ -1635,11 +1649,15 @@ void run_ghost_sync(State& s) {
     const int nb = nblocks(NA, kThreads);
     prof_begin(K_GHOST_SYNC);
     if (s.ghost_exact) {
-        if (s.precision == 1) k_ghost_sync<2, true><<<nb, kThreads, 0, s.stream>>>(po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
-        else k_ghost_sync<2, false><<<nb, kThreads, 0, s.stream>>>(po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
+        if (s.precision == 1) launch(s, nb, kThreads, 0, (k_ghost_sync<2, true>), po, pn, p32o, p32n, s.vel.b[s.vc],
+                                     s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
+        else launch(s, nb, kThreads, 0, (k_ghost_sync<2, false>), po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed,
+                    s.rbk, s.gsrc, s.groot, s.gcode, a);
     } else {
-        if (s.precision == 1) k_ghost_sync<1, true><<<nb, kThreads, 0, s.stream>>>(po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
-        else k_ghost_sync<1, false><<<nb, kThreads, 0, s.stream>>>(po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
+        if (s.precision == 1) launch(s, nb, kThreads, 0, (k_ghost_sync<1, true>), po, pn, p32o, p32n, s.vel.b[s.vc],
+                                     s.dem_fixed, s.rbk, s.gsrc, s.groot, s.gcode, a);
+        else launch(s, nb, kThreads, 0, (k_ghost_sync<1, false>), po, pn, p32o, p32n, s.vel.b[s.vc], s.dem_fixed,
+                    s.rbk, s.gsrc, s.groot, s.gcode, a);
     }
     launched(K_GHOST_SYNC);
     prof_end(K_GHOST_SYNC);
@@ -1658,11 +1676,15 @@ void run_final(State& s, double dt) {
     prof_begin(K_FINAL);
     const double h = 0.5 * dt;
     if (s.precision == 1) {
-        if (thermo) k_final<true, true><<<nb, kThreads, 0, s.stream>>>(s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part, N, h);
-        else k_final<true, false><<<nb, kThreads, 0, s.stream>>>(s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part, N, h);
+        if (thermo) launch(s, nb, kThreads, 0, (k_final<true, true>), s.vel.b[s.vc], s.frc.b[s.ac], s.frc32,
+                           s.red_part, N, h);
+        else launch(s, nb, kThreads, 0, (k_final<true, false>), s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part, N,
+                    h);
     } else {
-        if (thermo) k_final<false, true><<<nb, kThreads, 0, s.stream>>>(s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part, N, h);
-        else k_final<false, false><<<nb, kThreads, 0, s.stream>>>(s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part, N, h);
+        if (thermo) launch(s, nb, kThreads, 0, (k_final<false, true>), s.vel.b[s.vc], s.frc.b[s.ac], s.frc32,
+                           s.red_part, N, h);
+        else launch(s, nb, kThreads, 0, (k_final<false, false>), s.vel.b[s.vc], s.frc.b[s.ac], s.frc32, s.red_part,
+                    N, h);
     }
     launched(K_FINAL);
     prof_end(K_FINAL);
@@ -1674,7 +1696,7 @@ void run_refresh_pos32(State& s) {
     const int NA = s.N + s.G;
     if (NA == 0) return;
     StepArgs a = step_args(s, 0.0);
-    k_refresh_pos32<<<nblocks(NA, kThreads), kThreads, 0, s.stream>>>(s.pos.b[s.pc], s.pos32.b[s.pc], s.rbk, NA, a);
+    launch(s, nblocks(NA, kThreads), kThreads, 0, k_refresh_pos32, s.pos.b[s.pc], s.pos32.b[s.pc], s.rbk, NA, a);
     launched(K_MISC);
 }
 
@@ -1682,8 +1704,8 @@ long long count_pairs_inside(State& s, double rc) {
     if (s.N == 0 || !s.lists_valid) return 0;
     unsigned long long* d = reinterpret_cast<unsigned long long*>(s.thermo_dev + 6);  // spare words
     TMD_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned long long), s.stream));
-    k_count_inside<<<nblocks(s.N, kThreads), kThreads, 0, s.stream>>>(s.pos.b[s.pc], s.nbn, s.nbl, s.N, s.nb_stride,
-                                                                      s.nb_cap, rc * rc, d);
+    launch(s, nblocks(s.N, kThreads), kThreads, 0, k_count_inside, s.pos.b[s.pc], s.nbn, s.nbl, s.N, s.nb_stride,
+           s.nb_cap, rc * rc, d);
     launched(K_MISC);
     unsigned long long h = 0;
     TMD_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, s.stream));
