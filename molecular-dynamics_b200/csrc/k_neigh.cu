@@ -1429,6 +1429,7 @@ static int finish_build(State& s, bool half) {
     s.cells_filled = s.status_host->filled;
     s.img_ok = (s.status_host->img_over1 == 0 ? 1 : 0) | (s.status_host->img_over2 == 0 ? 2 : 0);
     const int mx = s.status_host->max_nb;
+    s.max_list = mx;
     if (mx <= s.nb_cap) {
         s.lists_valid = 1;
         s.lists_half = half;

@@ -914,37 +914,84 @@ __device__ __forceinline__ void dem_pair(const double4& del, double rsq, const d
     for (int d = 0; d < 3; ++d) out[d] = dsub(dmul(n[d], fn), dmul(dmul(vt[d], tinv), ft));
 }
 
-template <bool HALF>
+// TWO_PASS (full lists): the entries in contact are found first, a list quad's four positions at a time,
+// and queued in shared memory; their forces follow, each contact's position and velocity loading while
+// the one before runs.  For lists with many entries out of contact: there a warp's lanes meet their
+// contacts at different entries, and the long pair force ran for a few lanes at a time.
+constexpr int kTouchQueue = 16;
+
+template <bool HALF, bool TWO_PASS = false>
 __global__ void __launch_bounds__(kThreads)
 k_dem_fp64(const double4* __restrict__ pos, const double4* __restrict__ vel, double4* __restrict__ frc,
            const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot, DemArgs a) {
     const int blk = (int)blockIdx.x + pdl_wait();
+    __shared__ int s_touch[TWO_PASS ? kTouchQueue : 1][kThreads];
     const int i = blk * blockDim.x + threadIdx.x;
     if (i >= a.N) return;
-    const double4 pi = pos[i];
-    const double4 vi = vel[i];
+    const double4 pi = ldg_d4(pos + i);
+    const double4 vi = ldg_d4(vel + i);
     // the reference closure's pair force is exactly zero (r < 2R gives sqrt(r^2) <= 2R, so its
     // penetration test never passes): the loop would only add +0.0
     const int n = a.fixed ? min(nbn[i], a.nbcap) : 0;
     double F[3] = {0.0, 0.0, 0.0};
-    uint4 eq = make_uint4(0u, 0u, 0u, 0u);
-    for (int k = 0; k < n; ++k) {
-        if ((k & 3) == 0) eq = list_quad(nbl, k >> 2, i, a.stride);
-        const int j = (int)((k & 2 ? (k & 1 ? eq.w : eq.z) : (k & 1 ? eq.y : eq.x)) >> kCodeBits);
-        const double4 pj = ldg_d4(pos + j);
-        const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
-        const double rsq = len2_strict(del.x, del.y, del.z);
-        if (rsq < a.rc2) {
-            double f[3];
-            dem_pair(del, rsq, vi, ldg_d4(vel + j), a, f);
-            F[0] = dadd(F[0], f[0]);
-            F[1] = dadd(F[1], f[1]);
-            F[2] = dadd(F[2], f[2]);
-            if (HALF) {
-                const int t = reaction_slot(j, a.N, groot);
-                atomicAdd(&frc[t].x, -f[0]);
-                atomicAdd(&frc[t].y, -f[1]);
-                atomicAdd(&frc[t].z, -f[2]);
+    if constexpr (TWO_PASS) {
+        const double d2 = dmul(a.radius, 2.0), touch2 = dmul(d2, d2);
+        const int nq = (n + 3) >> 2;
+        uint4 eq = n > 0 ? list_quad(nbl, 0, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        for (int b = 0; b < nq;) {
+            int c = 0;
+            for (; b < nq && c <= kTouchQueue - 4; ++b) {
+                const int j[4] = {(int)(eq.x >> kCodeBits), (int)(eq.y >> kCodeBits), (int)(eq.z >> kCodeBits),
+                                  (int)(eq.w >> kCodeBits)};
+                double4 pj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) pj[u] = ldg_d4(pos + j[u]);
+                if (b + 1 < nq) eq = list_quad(nbl, b + 1, i, a.stride);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const double rsq = len2_strict(dsub(pi.x, pj[u].x), dsub(pi.y, pj[u].y), dsub(pi.z, pj[u].z));
+                    // beyond the contact distance the pair force is exactly zero
+                    const bool touch = 4 * b + u < n && rsq < a.rc2 && rsq < touch2;
+                    if (touch) s_touch[c][threadIdx.x] = j[u];
+                    c += touch ? 1 : 0;
+                }
+            }
+            if (c == 0) continue;
+            int j = s_touch[0][threadIdx.x];
+            double4 pn = ldg_d4(pos + j), vn = ldg_d4(vel + j);
+            for (int q = 0; q < c; ++q) {
+                const double4 pj = pn, vj = vn;
+                j = s_touch[min(q + 1, c - 1)][threadIdx.x];
+                pn = ldg_d4(pos + j);
+                vn = ldg_d4(vel + j);
+                const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
+                double f[3];
+                dem_pair(del, len2_strict(del.x, del.y, del.z), vi, vj, a, f);
+                F[0] = dadd(F[0], f[0]);
+                F[1] = dadd(F[1], f[1]);
+                F[2] = dadd(F[2], f[2]);
+            }
+        }
+    } else {
+        uint4 eq = make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < n; ++k) {
+            if ((k & 3) == 0) eq = list_quad(nbl, k >> 2, i, a.stride);
+            const int j = (int)((k & 2 ? (k & 1 ? eq.w : eq.z) : (k & 1 ? eq.y : eq.x)) >> kCodeBits);
+            const double4 pj = ldg_d4(pos + j);
+            const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
+            const double rsq = len2_strict(del.x, del.y, del.z);
+            if (rsq < a.rc2) {
+                double f[3];
+                dem_pair(del, rsq, vi, ldg_d4(vel + j), a, f);
+                F[0] = dadd(F[0], f[0]);
+                F[1] = dadd(F[1], f[1]);
+                F[2] = dadd(F[2], f[2]);
+                if (HALF) {
+                    const int t = reaction_slot(j, a.N, groot);
+                    atomicAdd(&frc[t].x, -f[0]);
+                    atomicAdd(&frc[t].y, -f[1]);
+                    atomicAdd(&frc[t].z, -f[2]);
+                }
             }
         }
     }
@@ -955,6 +1002,55 @@ k_dem_fp64(const double4* __restrict__ pos, const double4* __restrict__ vel, dou
     } else {
         frc[i] = make_double4(F[0], F[1], F[2], 0.0);
     }
+}
+
+// Few grains (full lists): L lanes to a grain, lane `sub` taking entries sub, sub + L, ..., so that the
+// long pair forces of a grain run side by side.  Bit-identical to k_dem_fp64: the lanes put a round's
+// forces into shared memory and three of them add one component each in list order (an entry out of
+// contact adds +0.0, which changes no bit of a sum that starts at +0.0).
+template <int L>
+__global__ void __launch_bounds__(kThreads)
+k_dem_fp64_lanes(const double4* __restrict__ pos, const double4* __restrict__ vel, double4* __restrict__ frc,
+                 const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, DemArgs a) {
+    static_assert(L >= 4, "three lanes of a grain add its force's components");
+    const int blk = (int)blockIdx.x + pdl_wait();
+    __shared__ double s_f[3][kThreads + 4];
+    const int t = blk * kThreads + threadIdx.x;
+    const int i = t / L, sub = t % L;
+    const int n = i < a.N && a.fixed ? min(nbn[i], a.nbcap) : 0;
+    const int ic = i < a.N ? i : 0;
+    const double4 pi = ldg_d4(pos + ic), vi = ldg_d4(vel + ic);
+    const int rounds = __reduce_max_sync(0xffffffffu, (n + L - 1) / L);
+    double acc = 0.0;  // component `sub` of the force (sub < 3)
+    // the position of the next round's entry loads while this one's force runs
+    auto slot = [&](int k) { return k < n ? (int)(__ldg(nbl + nl_index(k, ic, a.stride)) >> kCodeBits) : ic; };
+    int jn = slot(sub), jnn = slot(sub + L);
+    double4 pn = ldg_d4(pos + jn);
+    for (int r = 0; r < rounds; ++r) {
+        const int k = r * L + sub, j = jn;
+        const double4 pj = pn;
+        jn = jnn;
+        pn = ldg_d4(pos + jn);
+        jnn = slot(k + 2 * L);
+        const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
+        const double rsq = len2_strict(del.x, del.y, del.z);
+        double f[3] = {0.0, 0.0, 0.0};
+        if (k < n && rsq < a.rc2) dem_pair(del, rsq, vi, ldg_d4(vel + j), a, f);
+        s_f[0][threadIdx.x] = f[0];
+        s_f[1][threadIdx.x] = f[1];
+        s_f[2][threadIdx.x] = f[2];
+        __syncwarp();
+        if (sub < 3) {
+            const double* q = s_f[sub] + (threadIdx.x - sub);
+#pragma unroll
+            for (int e = 0; e < L; ++e) acc = dadd(acc, q[e]);
+        }
+        __syncwarp();
+    }
+    const int base = (threadIdx.x & 31) - sub;
+    const double fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
+                 fz = __shfl_sync(0xffffffffu, acc, base + 2);
+    if (i < a.N && sub == 0) frc[i] = make_double4(fx, fy, fz, 0.0);
 }
 
 // Mixed DEM: the contact-fixed model's pair force in FP32 (same expression order
@@ -968,6 +1064,72 @@ struct DemMixedArgs {
     float hx, hy, hz;                    // rebasing shift decode scales (as k_lj_mixed_bf)
 };
 
+// One list entry: its force on i is added to f (FP32), or near a decision to c (FP64 pair); for a half
+// list the reaction goes to the neighbour's root.
+template <bool HALF>
+__device__ __forceinline__ void dem_mixed_pair(uint32_t en, int i, const float4& ri, const float4& rj,
+                                               const double4& vd, const float3& vi,
+                                               const double4* __restrict__ pos,
+                                               const double4* __restrict__ vel, float4* __restrict__ frc32,
+                                               const int* __restrict__ groot, const DemArgs& a,
+                                               const DemMixedArgs& b, float* f, double* c) {
+    const int j = (int)(en >> kCodeBits);
+    const float sx = __int_as_float((int)((en & 0x03u) | 0x4B000000u)) - 8388609.0f;
+    const float sy = __int_as_float((int)((en & 0x0Cu) | 0x4B000000u)) - 8388612.0f;
+    const float sz = __int_as_float((int)((en & 0x30u) | 0x4B000000u)) - 8388624.0f;
+    const float dx = fmaf(b.hx, sx, ri.x - rj.x);
+    const float dy = fmaf(b.hy, sy, ri.y - rj.y);
+    const float dz = fmaf(b.hz, sz, ri.z - rj.z);
+    const float rsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (!(rsq < b.rc2_hi) || !(rsq < b.c2_hi)) return;  // beyond the cutoff or no contact
+    if (rsq >= b.rc2_lo || rsq >= b.c2_lo) {
+        // near a decision: the FP64 pair
+        const double4 pi = pos[i], pj = pos[j];
+        const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
+        const double r2 = len2_strict(del.x, del.y, del.z);
+        if (r2 < a.rc2) {
+            double o[3];
+            dem_pair(del, r2, vd, ldg_d4(vel + j), a, o);
+            c[0] += o[0];
+            c[1] += o[1];
+            c[2] += o[2];
+            if (HALF) {
+                const int t = reaction_slot(j, a.N, groot);
+                add_force32(frc32 + t, (float)(-o[0]), (float)(-o[1]), (float)(-o[2]));
+            }
+        }
+        return;
+    }
+    const double4 vj = ldg_d4(vel + j);
+    // |del| and 1/|del| from one reciprocal square root (against a rounded square root and
+    // a division: the force 33.0 -> 28.9 us on the 48^3 FCC split)
+    if (!(rsq > 0.f)) return;
+    const float inv = rsqrtf(rsq);
+    const float len = rsq * inv;
+    const float delta = b.d2 - len;
+    const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
+    const float rvx = vi.x - (float)vj.x, rvy = vi.y - (float)vj.y, rvz = vi.z - (float)vj.z;
+    const float vn = rvx * nx + rvy * ny + rvz * nz;
+    const float vtx = rvx - nx * vn, vty = rvy - ny * vn, vtz = rvz - nz * vn;
+    const float vt2 = vtx * vtx + vty * vty + vtz * vtz;
+    const float tinv = vt2 > 0.f ? rsqrtf(vt2) : 0.f;
+    const float vtl = vt2 * tinv;
+    float fn = b.k * delta - b.dn * vn;
+    if (fn < 0.f) fn = 0.f;
+    const float t1 = b.dt_ * vtl, t2 = b.mu * fn;
+    const float ft = t1 < t2 ? t1 : t2;
+    const float px = nx * fn - vtx * tinv * ft;
+    const float py = ny * fn - vty * tinv * ft;
+    const float pz = nz * fn - vtz * tinv * ft;
+    f[0] += px;
+    f[1] += py;
+    f[2] += pz;
+    if (HALF) {
+        const int t = reaction_slot(j, a.N, groot);
+        add_force32(frc32 + t, -px, -py, -pz);
+    }
+}
+
 template <bool HALF>
 __global__ void __launch_bounds__(kThreads)
 k_dem_mixed(const float4* __restrict__ pos32, const double4* __restrict__ pos, const double4* __restrict__ vel,
@@ -976,81 +1138,65 @@ k_dem_mixed(const float4* __restrict__ pos32, const double4* __restrict__ pos, c
     const int blk = (int)blockIdx.x + pdl_wait();
     const int i = blk * blockDim.x + threadIdx.x;
     if (i >= a.N) return;
-    float fx = 0.f, fy = 0.f, fz = 0.f;
-    double cx = 0.0, cy = 0.0, cz = 0.0;
+    float f[3] = {0.f, 0.f, 0.f};
+    double c[3] = {0.0, 0.0, 0.0};
     if (a.fixed) {
         const float4 ri = pos32[i];
-        const double4 vi = vel[i];
-        const float vix = (float)vi.x, viy = (float)vi.y, viz = (float)vi.z;
+        const double4 v = vel[i];
+        const float3 vi = make_float3((float)v.x, (float)v.y, (float)v.z);
         const int n = min(nbn[i], a.nbcap);
         uint4 eq = make_uint4(0u, 0u, 0u, 0u);
         for (int k = 0; k < n; ++k) {
             if ((k & 3) == 0) eq = list_quad(nbl, k >> 2, i, a.stride);
             const uint32_t en = k & 2 ? (k & 1 ? eq.w : eq.z) : (k & 1 ? eq.y : eq.x);
-            const int j = (int)(en >> kCodeBits);
-            const float4 rj = __ldg(pos32 + j);
-            const float sx = __int_as_float((int)((en & 0x03u) | 0x4B000000u)) - 8388609.0f;
-            const float sy = __int_as_float((int)((en & 0x0Cu) | 0x4B000000u)) - 8388612.0f;
-            const float sz = __int_as_float((int)((en & 0x30u) | 0x4B000000u)) - 8388624.0f;
-            const float dx = fmaf(b.hx, sx, ri.x - rj.x);
-            const float dy = fmaf(b.hy, sy, ri.y - rj.y);
-            const float dz = fmaf(b.hz, sz, ri.z - rj.z);
-            const float rsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            if (!(rsq < b.rc2_hi) || !(rsq < b.c2_hi)) continue;  // beyond the cutoff or no contact
-            if (rsq >= b.rc2_lo || rsq >= b.c2_lo) {
-                // near a decision: the FP64 pair
-                const double4 pi = pos[i], pj = pos[j];
-                const double4 del = make_double4(dsub(pi.x, pj.x), dsub(pi.y, pj.y), dsub(pi.z, pj.z), 0.0);
-                const double r2 = len2_strict(del.x, del.y, del.z);
-                if (r2 < a.rc2) {
-                    double o[3];
-                    dem_pair(del, r2, vi, ldg_d4(vel + j), a, o);
-                    cx += o[0];
-                    cy += o[1];
-                    cz += o[2];
-                    if (HALF) {
-                        const int t = reaction_slot(j, a.N, groot);
-                        add_force32(frc32 + t, (float)(-o[0]), (float)(-o[1]), (float)(-o[2]));
-                    }
-                }
-                continue;
-            }
-            const double4 vj = ldg_d4(vel + j);
-            // |del| and 1/|del| from one reciprocal square root (against a rounded square root and
-            // a division: the force 33.0 -> 28.9 us on the 48^3 FCC split)
-            if (!(rsq > 0.f)) continue;
-            const float inv = rsqrtf(rsq);
-            const float len = rsq * inv;
-            const float delta = b.d2 - len;
-            const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
-            const float rvx = vix - (float)vj.x, rvy = viy - (float)vj.y, rvz = viz - (float)vj.z;
-            const float vn = rvx * nx + rvy * ny + rvz * nz;
-            const float vtx = rvx - nx * vn, vty = rvy - ny * vn, vtz = rvz - nz * vn;
-            const float vt2 = vtx * vtx + vty * vty + vtz * vtz;
-            const float tinv = vt2 > 0.f ? rsqrtf(vt2) : 0.f;
-            const float vtl = vt2 * tinv;
-            float fn = b.k * delta - b.dn * vn;
-            if (fn < 0.f) fn = 0.f;
-            const float t1 = b.dt_ * vtl, t2 = b.mu * fn;
-            const float ft = t1 < t2 ? t1 : t2;
-            const float px = nx * fn - vtx * tinv * ft;
-            const float py = ny * fn - vty * tinv * ft;
-            const float pz = nz * fn - vtz * tinv * ft;
-            fx += px;
-            fy += py;
-            fz += pz;
-            if (HALF) {
-                const int t = reaction_slot(j, a.N, groot);
-                add_force32(frc32 + t, -px, -py, -pz);
-            }
+            dem_mixed_pair<HALF>(en, i, ri, __ldg(pos32 + (en >> kCodeBits)), v, vi, pos, vel, frc32, groot, a, b, f, c);
         }
     }
-    const float Fx = (float)((double)fx + cx), Fy = (float)((double)fy + cy), Fz = (float)((double)fz + cz);
+    const float Fx = (float)((double)f[0] + c[0]), Fy = (float)((double)f[1] + c[1]), Fz = (float)((double)f[2] + c[2]);
     if (HALF) {
         add_force32(frc32 + i, Fx, Fy, Fz);
     } else {
         frc32[i] = make_float4(Fx, Fy, Fz, 0.f);
     }
+}
+
+// few grains, L lanes to a grain (see k_dem_fp64_lanes); the lanes' sums are added in FP64
+template <int L>
+__global__ void __launch_bounds__(kThreads)
+k_dem_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ pos, const double4* __restrict__ vel,
+                  float4* __restrict__ frc32, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, DemArgs a,
+                  DemMixedArgs b) {
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int t = blk * kThreads + threadIdx.x;
+    const int i = t / L, sub = t % L;
+    float f[3] = {0.f, 0.f, 0.f};
+    double c[3] = {0.0, 0.0, 0.0};
+    if (i < a.N && a.fixed) {
+        const float4 ri = pos32[i];
+        const double4 v = ldg_d4(vel + i);
+        const float3 vi = make_float3((float)v.x, (float)v.y, (float)v.z);
+        const int n = min(nbn[i], a.nbcap);
+        uint32_t en = sub < n ? __ldg(nbl + nl_index(sub, i, a.stride)) : 0u;
+        float4 rn = __ldg(pos32 + (en >> kCodeBits));
+        for (int k = sub; k < n; k += L) {
+            const uint32_t e0 = en;
+            const float4 rj = rn;
+            if (k + L < n) {
+                en = __ldg(nbl + nl_index(k + L, i, a.stride));
+                rn = __ldg(pos32 + (en >> kCodeBits));
+            }
+            dem_mixed_pair<false>(e0, i, ri, rj, v, vi, pos, vel, frc32, nullptr, a, b, f, c);
+        }
+    }
+    double F[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) F[d] = (double)f[d] + c[d];
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) F[d] += __shfl_xor_sync(0xffffffffu, F[d], o);
+    if (i < a.N && sub == 0) frc32[i] = make_float4((float)F[0], (float)F[1], (float)F[2], 0.f);
 }
 
 // ---- integration + ghost refresh ------------------------------------------------
@@ -1538,6 +1684,28 @@ void run_ghost_refresh(State& s, int gm) {
     prof_end(K_GHOST_SYNC);
 }
 
+// Lanes per grain of a full-list DEM force kernel, and the two-pass FP64 kernel.  Lists of up to 12
+// entries (the kissing number of equal spheres) are taken as beds whose neighbours all touch, longer
+// ones as having entries out of contact (granular gas: 18 entries, 6 contacts).  Step times in us
+// (contact model, rebuild every 20 steps included), thread per grain / two-pass / 4 lanes / 8 lanes:
+//   FP64 gas  4,000 grains 17.7 / 11.5 / 10.4 / 9.6   18,377  20.5 / 13.6 / 11.5 / 12.3
+//            32,000        21.8 / 15.0 / 14.1 / 15.6  52,740  23.3 / 16.8 / 19.3 / 21.5
+//           110,700        28.4 / 29.6 / 31.6        152,065  36.9 / 33.8 / 41.1   260,800 52.5 / 48.8 / 65.2
+//   FP64 bed 28,224        16.9 / 15.2 / 11.7 / 14.2  66,560  20.1 / 20.2 / 19.2   223,488 40.5 / 48.6 / 45.9
+//   mixed gas 4,000        16.0 / -    /  9.7 /  8.4  52,740  19.4 / -    / 16.2    77,598 20.3 / -    / 20.6
+//   mixed bed 28,224       16.6 / -    / 10.9 / 12.7  66,560  19.0 / -    / 18.0    94,608 20.3 / -    / 22.0
+static int dem_lanes(const State& s) {
+    if (s.N <= 12000) return 8;
+    return s.N <= (s.precision == 1 ? 64000 : s.max_list > 12 ? 36000 : 72000) ? 4 : 1;
+}
+
+// the two-pass kernel's registers hold five blocks per SM, the other's eight: between one wave of the
+// former and one of the latter (94,720 to 151,552 grains) a second wave costs more than it saves
+static bool dem_two_pass(const State& s) {
+    constexpr int kTwoPassWave = 148 * 5 * kThreads, kWave = 148 * 8 * kThreads;
+    return s.max_list > 12 && !(s.N > kTwoPassWave && s.N <= kWave);
+}
+
 void run_force_dem(State& s, const PendingForce& p) {
     const int N = s.N;
     if (N == 0) return;
@@ -1573,12 +1741,20 @@ void run_force_dem(State& s, const PendingForce& p) {
             launched(K_MISC);
         }
         prof_begin(K_FORCE_DEM);
+        const int lanes = p.half ? 1 : dem_lanes(s);
+        const int nb = nblocks((long long)N * lanes, kThreads);
         if (p.half)
-            launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_mixed<true>, s.pos32.b[s.pc], s.pos.b[s.pc],
-                   s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
+            launch(s, nb, kThreads, 0, k_dem_mixed<true>, s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32, s.nbn,
+                   s.nbl, s.groot, a, b);
+        else if (lanes == 8)
+            launch(s, nb, kThreads, 0, k_dem_mixed_lanes<8>, s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32,
+                   s.nbn, s.nbl, a, b);
+        else if (lanes == 4)
+            launch(s, nb, kThreads, 0, k_dem_mixed_lanes<4>, s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32,
+                   s.nbn, s.nbl, a, b);
         else
-            launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_mixed<false>, s.pos32.b[s.pc], s.pos.b[s.pc],
-                   s.vel.b[s.vc], s.frc32, s.nbn, s.nbl, s.groot, a, b);
+            launch(s, nb, kThreads, 0, k_dem_mixed<false>, s.pos32.b[s.pc], s.pos.b[s.pc], s.vel.b[s.vc], s.frc32, s.nbn,
+                   s.nbl, s.groot, a, b);
         launched(K_FORCE_DEM);
         prof_end(K_FORCE_DEM);
         return;
@@ -1588,12 +1764,19 @@ void run_force_dem(State& s, const PendingForce& p) {
         launched(K_MISC);
     }
     prof_begin(K_FORCE_DEM);
+    const int lanes = p.half ? 1 : dem_lanes(s);
+    const int nb = nblocks((long long)N * lanes, kThreads);
+    const double4 *pos = s.pos.b[s.pc], *vel = s.vel.b[s.vc];
     if (p.half)
-        launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_fp64<true>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
-               s.nbn, s.nbl, s.groot, a);
+        launch(s, nb, kThreads, 0, k_dem_fp64<true>, pos, vel, s.frc.b[s.ac], s.nbn, s.nbl, s.groot, a);
+    else if (lanes == 8)
+        launch(s, nb, kThreads, 0, k_dem_fp64_lanes<8>, pos, vel, s.frc.b[s.ac], s.nbn, s.nbl, a);
+    else if (lanes == 4)
+        launch(s, nb, kThreads, 0, k_dem_fp64_lanes<4>, pos, vel, s.frc.b[s.ac], s.nbn, s.nbl, a);
+    else if (dem_two_pass(s))
+        launch(s, nb, kThreads, 0, (k_dem_fp64<false, true>), pos, vel, s.frc.b[s.ac], s.nbn, s.nbl, s.groot, a);
     else
-        launch(s, nblocks(N, kThreads), kThreads, 0, k_dem_fp64<false>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
-               s.nbn, s.nbl, s.groot, a);
+        launch(s, nb, kThreads, 0, k_dem_fp64<false>, pos, vel, s.frc.b[s.ac], s.nbn, s.nbl, s.groot, a);
     launched(K_FORCE_DEM);
     prof_end(K_FORCE_DEM);
 }

@@ -169,6 +169,7 @@ struct State {
     int nblk_border = 0;
     int lists_valid = 0;
     bool lists_half = false;
+    int max_list = 0;      // longest list of the last build whose status was read
     int cells_filled = 0;  // cells that hold locals, at the last binning whose status was read (0: none)
 
     // modes
