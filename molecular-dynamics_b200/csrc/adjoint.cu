@@ -106,8 +106,8 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
     double ux = 0.0, uy = 0.0, uz = 0.0, Fx = 0.0, Fy = 0.0, Fz = 0.0, gs = 0.0;
     double4 wi = make_double4(0.0, 0.0, 0.0, 0.0);
     if (act) {
-        const double4 xi = xs[i];
-        wi = w[i];
+        const double4 xi = ldg_d4(xs + i);
+        wi = ldg_d4(w + i);
         const int n = min(nbn[i], a.nbcap);
         int ej[kHb], er[kHb];
 #pragma unroll
@@ -165,12 +165,12 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
     double ge = 0.0;
     if (act && sub == 0) {
         ge = (wi.x * Fx + wi.y * Fy + wi.z * Fz) / a.eps;
-        double4 q = ax[i];
+        double4 q = ld_d4(ax + i);
         q.x += a.kick * ux;
         q.y += a.kick * uy;
         q.z += a.kick * uz;
-        ax[i] = q;
-        w_next[i] = make_double4(wi.x + a.drift * q.x, wi.y + a.drift * q.y, wi.z + a.drift * q.z, 0.0);
+        st_d4(ax + i, q);
+        st_d4(w_next + i, make_double4(wi.x + a.drift * q.x, wi.y + a.drift * q.y, wi.z + a.drift * q.z, 0.0));
     }
     const double se = block_sum(ge, scratch);
     const double ss = block_sum(gs, scratch);
@@ -288,14 +288,14 @@ __global__ void k_to_ref(const double4* __restrict__ src, const int* __restrict_
                          int N) {
     const int blk = (int)blockIdx.x + pdl_wait();
     const int s = blk * blockDim.x + threadIdx.x;
-    if (s < N) dst[ref[s]] = src[s];
+    if (s < N) st_d4(dst + ref[s], ldg_d4(src + s));
 }
 // reference order -> slot order (locals)
 __global__ void k_from_ref(const double4* __restrict__ src, const int* __restrict__ ref, double4* __restrict__ dst,
                            int N) {
     const int blk = (int)blockIdx.x + pdl_wait();
     const int s = blk * blockDim.x + threadIdx.x;
-    if (s < N) dst[s] = src[ref[s]];
+    if (s < N) st_d4(dst + s, ldg_d4(src + ref[s]));
 }
 // checkpoint of the current state in reference order
 __global__ void k_checkpoint(const double4* __restrict__ pos, const double4* __restrict__ vel,
@@ -305,8 +305,8 @@ __global__ void k_checkpoint(const double4* __restrict__ pos, const double4* __r
     const int s = blk * blockDim.x + threadIdx.x;
     if (s < N) {
         const int r = ref[s];
-        cx[r] = pos[s];
-        cv[r] = vel[s];
+        st_d4(cx + r, ldg_d4(pos + s));
+        st_d4(cv + r, ldg_d4(vel + s));
         ci[r] = img[s];
     }
 }
@@ -318,8 +318,8 @@ __global__ void k_restore(const double4* __restrict__ cx, const double4* __restr
     const int blk = (int)blockIdx.x + pdl_wait();
     const int r = blk * blockDim.x + threadIdx.x;
     if (r < N) {
-        pos[r] = cx[r];
-        vel[r] = cv[r];
+        st_d4(pos + r, ldg_d4(cx + r));
+        st_d4(vel + r, ldg_d4(cv + r));
         img[r] = ci[r];
         ref[r] = r;
         slot_of_ref[r] = r;

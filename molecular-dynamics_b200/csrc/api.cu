@@ -605,12 +605,12 @@ __global__ void k_gather_ref(const double4* __restrict__ pos, const double4* __r
     double* ov = out + 4 * (size_t)NA;
     double* of = out + 7 * (size_t)NA;
     om[r] = mass[slot];
-    const double4 p = pos[slot];
+    const double4 p = ldg_d4(pos + slot);
     op[3 * (size_t)r] = p.x;
     op[3 * (size_t)r + 1] = p.y;
     op[3 * (size_t)r + 2] = p.z;
     double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (r < N || ghost_vel) v = vel[slot];
+    if (r < N || ghost_vel) v = ldg_d4(vel + slot);
     ov[3 * (size_t)r] = v.x;
     ov[3 * (size_t)r + 1] = v.y;
     ov[3 * (size_t)r + 2] = v.z;
@@ -620,7 +620,7 @@ __global__ void k_gather_ref(const double4* __restrict__ pos, const double4* __r
             const float4 f = frc32[slot];
             fx = f.x, fy = f.y, fz = f.z;
         } else {
-            const double4 f = frc[slot];
+            const double4 f = ldg_d4(frc + slot);
             fx = f.x, fy = f.y, fz = f.z;
         }
     }
@@ -639,9 +639,9 @@ __global__ void k_upload(const double* __restrict__ m, const double* __restrict_
     const int i = blk * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const size_t k = 3 * (size_t)i;
-    pos[i] = make_double4(p[k], p[k + 1], p[k + 2], 0.0);
-    vel[i] = make_double4(v[k], v[k + 1], v[k + 2], 0.0);
-    frc[i] = make_double4(0.0, 0.0, 0.0, 0.0);
+    st_d4(pos + i, make_double4(p[k], p[k + 1], p[k + 2], 0.0));
+    st_d4(vel + i, make_double4(v[k], v[k + 1], v[k + 2], 0.0));
+    st_d4(frc + i, make_double4(0.0, 0.0, 0.0, 0.0));
     frc32[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     mass[i] = m[i];
     ref[i] = i;

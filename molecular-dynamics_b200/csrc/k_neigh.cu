@@ -88,7 +88,7 @@ __device__ __forceinline__ int rebase_cell(const double4& p, const GeoArgs& a) {
 // the world box.  img counts wraps so the adjoint can unwrap displacements.
 __device__ __forceinline__ double4 wrap_local(double4* __restrict__ pos, int* __restrict__ img, int i,
                                               const GeoArgs& a) {
-    double4 p = pos[i];
+    double4 p = ld_d4(pos + i);
     double c[3] = {p.x, p.y, p.z};
     int im = img[i];
     int w[3] = {unpack_axis(im, 0), unpack_axis(im, 1), unpack_axis(im, 2)};
@@ -99,7 +99,7 @@ __device__ __forceinline__ double4 wrap_local(double4* __restrict__ pos, int* __
         if (v > a.whi[d]) { c[d] = dsub(c[d], a.len[d]); w[d] += 1; }
     }
     p = make_double4(c[0], c[1], c[2], p.w);
-    pos[i] = p;
+    st_d4(pos + i, p);
     img[i] = pack3(w[0], w[1], w[2]);
     return p;
 }
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_count(double4* __rest
     unsigned m = 0;
     if (r < N) {
         const int sl = slot_of_ref[r];
-        m = border_mask(WRAP ? wrap_local(pos, img, sl, a) : pos[sl], a);
+        m = border_mask(WRAP ? wrap_local(pos, img, sl, a) : ld_d4(pos + sl), a);
         bmask[r] = m;
     }
     for (int t = 0; t < 26; ++t) {
@@ -218,9 +218,9 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
     __syncthreads();
     if (r >= N || (m & 0x03ffffffu) == 0) return;
     const int s_root = slot_of_ref[r];
-    const double4 p = pos[s_root];
+    const double4 p = ld_d4(pos + s_root);
     const double mroot = mass[s_root];
-    const double4 vroot = vel[s_root];
+    const double4 vroot = ld_d4(vel + s_root);
     const unsigned flags = m >> 26;
     // index of this root's ghost of type t (a type whose bit is set)
     auto gidx = [&](int t) { return boff[t * nblk + blk] + wpre[wid][t] + s_rank[t][threadIdx.x]; };
@@ -261,10 +261,10 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
             code |= (ls + 1) << (2 * d);
             code |= (tot[d] + 1) << (8 + 2 * d);
         }
-        pos[slot] = make_double4(c[0], c[1], c[2], 0.0);
+        st_d4(pos + slot, make_double4(c[0], c[1], c[2], 0.0));
         mass[slot] = mroot;
-        frc[slot] = make_double4(0.0, 0.0, 0.0, 0.0);
-        vel[slot] = sync_vel ? vroot : make_double4(0.0, 0.0, 0.0, 0.0);
+        st_d4(frc + slot, make_double4(0.0, 0.0, 0.0, 0.0));
+        st_d4(vel + slot, sync_vel ? vroot : make_double4(0.0, 0.0, 0.0, 0.0));
         ref[slot] = slot;
         slot_of_ref[slot] = slot;
         gsrc[g] = src_slot;
@@ -284,7 +284,7 @@ __global__ void k_bin_count(const double4* __restrict__ pos, int* __restrict__ c
     const int blk = (int)blockIdx.x + pdl_wait();
     int s = blk * blockDim.x + threadIdx.x;
     if (s >= NA) return;
-    int c = flat_cell(pos[s], a);
+    int c = flat_cell(ldg_d4(pos + s), a);
     if (c == a.ncells) atomicAdd(s < N ? &st->out_local : &st->out_ghost, 1);
     int seg = s < N ? c : (a.ncells + 1) + c;
     bin_cell[s] = c;
@@ -323,10 +323,11 @@ struct MoveArgs {
 
 __device__ __forceinline__ void move_slot(int n, int o, const MoveArgs& m, const GeoArgs& a) {
     m.slot_cell[n] = m.bin_cell[o];
-    const double4 p = m.pos_o[o];
-    m.pos_n[n] = p;
-    m.vel_n[n] = m.vel_o[o];
-    m.frc_n[n] = m.frc_o[o];
+    const double4 p = ldg_d4(m.pos_o + o);
+    const double4 v = ldg_d4(m.vel_o + o), f = ldg_d4(m.frc_o + o);
+    st_d4(m.pos_n + n, p);
+    st_d4(m.vel_n + n, v);
+    st_d4(m.frc_n + n, f);
     m.mass_n[n] = m.mass_o[o];
     const int r = m.ref_o[o];
     m.ref_n[n] = r;

@@ -135,7 +135,7 @@ __device__ __forceinline__ void write_ghost(int t, const double4& xs, int code, 
     x.y = dadd(xs.y, dmul(pa.len[1], (double)shift_axis(code, pa.base, 1)));
     x.z = dadd(xs.z, dmul(pa.len[2], (double)shift_axis(code, pa.base, 2)));
     x.w = 0.0;
-    pos_n[t] = x;
+    st_d4(pos_n + t, x);
     if (MIXED) pos32_n[t] = rebased32(x, pa.rbk[t], alo, rb_h);
 }
 
@@ -173,7 +173,7 @@ __device__ __forceinline__ void push_chain(int q, const double4* __restrict__ po
                                            double4* __restrict__ pos_n, float4* __restrict__ pos32_n,
                                            const double* alo, double rb_h) {
     const int h = pa.chain[q];
-    write_ghost<MIXED>(N + h, pos_o[pa.gsrc[h]], pa.gcode[h], pa, pos_n, pos32_n, alo, rb_h);
+    write_ghost<MIXED>(N + h, ldg_d4(pos_o + pa.gsrc[h]), pa.gcode[h], pa, pos_n, pos32_n, alo, rb_h);
 }
 
 // INIT (with FUSE, full lists): the epilogue also does the next step's initial integration
@@ -194,7 +194,7 @@ k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* _
     if (PUSH) prefetch_push(pa, a.N);
     double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
     if (i < a.N) {
-        const double4 pi = pos[i];
+        const double4 pi = ldg_d4(pos + i);
         double fx = 0.0, fy = 0.0, fz = 0.0;
         // quads of four entries; the next quad loads while this one's gathers are in flight
         // (entries past n are padding, skipped below)
@@ -242,9 +242,9 @@ k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* _
             atomicAdd(&frc[i].y, fy);
             atomicAdd(&frc[i].z, fz);
         } else {
-            frc[i] = make_double4(fx, fy, fz, 0.0);
+            st_d4(frc + i, make_double4(fx, fy, fz, 0.0));
             if (FUSE) {  // core/compute.impala:108-116
-                double4 v = vel[i];
+                double4 v = ld_d4(vel + i);
                 v.x = dadd(v.x, dmul(fx, a.h));
                 v.y = dadd(v.y, dmul(fy, a.h));
                 v.z = dadd(v.z, dmul(fz, a.h));
@@ -252,10 +252,10 @@ k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* _
                 if (INIT) {  // positions carry w = 0
                     double4 x = integrate_one(pi, v, fx, fy, fz, a.dt_i, a.h_i);
                     x.w = 0.0;
-                    pos_n[i] = x;
+                    st_d4(pos_n + i, x);
                     if (PUSH) push_images<false>(i, x, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
                 }
-                vel[i] = v;
+                st_d4(vel + i, v);
             }
         }
     } else if (PUSH && i < a.N + (pa.nchain_dev ? *pa.nchain_dev : pa.nchain)) {
@@ -589,7 +589,7 @@ k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos,
         const float4 F = make_float4((float)Fx, (float)Fy, (float)Fz, 0.f);
         frc32[i] = F;
         if (FUSE) {
-            double4 v = vel[i];
+            double4 v = ld_d4(vel + i);
             v.x += (double)F.x * a.h;
             v.y += (double)F.y * a.h;
             v.z += (double)F.z * a.h;
@@ -597,11 +597,11 @@ k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos,
             if (INIT) {
                 double4 x = integrate_one(ldg_d4(pos + i), v, (double)F.x, (double)F.y, (double)F.z, a.dt_i, a.h_i);
                 x.w = 0.0;  // positions carry w = 0
-                pos_n[i] = x;
+                st_d4(pos_n + i, x);
                 pos32_n[i] = rebased32(x, rbk[i], a.alo, a.rb_h);
                 if (PUSH) push_images<true>(i, x, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
             }
-            vel[i] = v;
+            st_d4(vel + i, v);
         }
         if (THERMO) {
             e += (double)ef;
@@ -724,7 +724,7 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
         const float4 F = make_float4((float)Fx, (float)Fy, (float)Fz, 0.f);
         if (act && sub == 0) frc32[i] = F;
         if (FUSE) {
-            double4 v = act ? vel[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+            double4 v = act ? ld_d4(vel + i) : make_double4(0.0, 0.0, 0.0, 0.0);
             v.x += (double)F.x * a.h;
             v.y += (double)F.y * a.h;
             v.z += (double)F.z * a.h;
@@ -733,13 +733,13 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
                 double4 x = integrate_one(ldg_d4(pos + i), v, (double)F.x, (double)F.y, (double)F.z, a.dt_i, a.h_i);
                 x.w = 0.0;  // positions carry w = 0
                 if (sub == 0) {
-                    pos_n[i] = x;
+                    st_d4(pos_n + i, x);
                     pos32_n[i] = rebased32(x, rbk[i], a.alo, a.rb_h);
                 }
                 if (PUSH) push_images_lanes<L, true>(i, sub, x, a.N, pa, pos_n, pos32_n, a.alo, a.rb_h);
             }
             __syncwarp();  // every lane has read the velocity
-            if (act && sub == 0) vel[i] = v;
+            if (act && sub == 0) st_d4(vel + i, v);
         }
         if (THERMO) {
             e += (double)ef;
@@ -787,7 +787,7 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
         const int i = t / L, sub = t % L, at = lane / L;
         const bool act = i < a.N;
         const int n = act ? min(nbn[i], a.nbcap) : 0;
-        const double4 pi = act ? pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        const double4 pi = act ? ldg_d4(pos + i) : make_double4(0.0, 0.0, 0.0, 0.0);
         double acc = 0.0;  // component `sub` of the force (sub < 3)
         const int nquad = (n + 3) >> 2;
         const int rounds = __reduce_max_sync(0xffffffffu, (nquad + L - 1) / L);
@@ -842,9 +842,9 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
         const int base = lane & ~(L - 1);
         const double fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
                      fz = __shfl_sync(0xffffffffu, acc, base + 2);
-        if (act && sub == 0) frc[i] = make_double4(fx, fy, fz, 0.0);
+        if (act && sub == 0) st_d4(frc + i, make_double4(fx, fy, fz, 0.0));
         if (FUSE) {  // core/compute.impala:108-116
-            double4 v = act ? vel[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+            double4 v = act ? ld_d4(vel + i) : make_double4(0.0, 0.0, 0.0, 0.0);
             v.x = dadd(v.x, dmul(fx, a.h));
             v.y = dadd(v.y, dmul(fy, a.h));
             v.z = dadd(v.z, dmul(fz, a.h));
@@ -852,11 +852,11 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
             if (INIT && act) {  // positions carry w = 0
                 double4 x = integrate_one(pi, v, fx, fy, fz, a.dt_i, a.h_i);
                 x.w = 0.0;
-                if (sub == 0) pos_n[i] = x;
+                if (sub == 0) st_d4(pos_n + i, x);
                 if (PUSH) push_images_lanes<L, false>(i, sub, x, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
             }
             __syncwarp();  // every lane has read the velocity
-            if (act && sub == 0) vel[i] = v;
+            if (act && sub == 0) st_d4(vel + i, v);
         }
     } else if (PUSH) {
         push_chain_block<false>(blk - atom_blocks, pos, a.N, pa, pos_n, nullptr, a.alo, a.rb_h);
@@ -1000,7 +1000,7 @@ k_dem_fp64(const double4* __restrict__ pos, const double4* __restrict__ vel, dou
         atomicAdd(&frc[i].y, F[1]);
         atomicAdd(&frc[i].z, F[2]);
     } else {
-        frc[i] = make_double4(F[0], F[1], F[2], 0.0);
+        st_d4(frc + i, make_double4(F[0], F[1], F[2], 0.0));
     }
 }
 
@@ -1050,7 +1050,7 @@ k_dem_fp64_lanes(const double4* __restrict__ pos, const double4* __restrict__ ve
     const int base = (threadIdx.x & 31) - sub;
     const double fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
                  fz = __shfl_sync(0xffffffffu, acc, base + 2);
-    if (i < a.N && sub == 0) frc[i] = make_double4(fx, fy, fz, 0.0);
+    if (i < a.N && sub == 0) st_d4(frc + i, make_double4(fx, fy, fz, 0.0));
 }
 
 // Mixed DEM: the contact-fixed model's pair force in FP32 (same expression order
@@ -1218,10 +1218,10 @@ template <bool MIXED>
 __device__ __forceinline__ void load_force(const double4* frc, const float4* frc32, int i, double& fx, double& fy,
                                            double& fz) {
     if (MIXED) {
-        const float4 f = frc32[i];
+        const float4 f = __ldg(frc32 + i);
         fx = f.x; fy = f.y; fz = f.z;
     } else {
-        const double4 f = frc[i];
+        const double4 f = ldg_d4(frc + i);
         fx = f.x; fy = f.y; fz = f.z;
     }
 }
@@ -1235,22 +1235,22 @@ k_integrate(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, cons
     const int blk = (int)blockIdx.x + pdl_wait();
     const int t = blk * blockDim.x + threadIdx.x;
     if (t < a.N) {
-        double4 v = vel_o[t];
+        double4 v = ldg_d4(vel_o + t);
         double fx, fy, fz;
         load_force<MIXED>(frc, frc32, t, fx, fy, fz);
         if (a.pre) kick(v, fx, fy, fz, a.hp);
-        const double4 x = integrate_one(pos_o[t], v, fx, fy, fz, a.dt, a.h);
-        pos_n[t] = x;
-        vel_n[t] = v;
+        const double4 x = integrate_one(ldg_d4(pos_o + t), v, fx, fy, fz, a.dt, a.h);
+        st_d4(pos_n + t, x);
+        st_d4(vel_n + t, v);
         if (MIXED) pos32_n[t] = rebased32(x, rbk[t], a.alo, a.rb_h);
         return;
     }
     if (t >= a.N + a.G) return;
     const int g = t - a.N;
     if (GM == 0) {
-        pos_n[t] = pos_o[t];
+        st_d4(pos_n + t, ldg_d4(pos_o + t));
         if (MIXED) pos32_n[t] = pos32_o[t];
-        if (DEMV) vel_n[t] = vel_o[t];
+        if (DEMV) st_d4(vel_n + t, ldg_d4(vel_o + t));
         return;
     }
     const int s = GM == 1 ? gsrc[g] : groot[g];
@@ -1258,13 +1258,13 @@ k_integrate(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, cons
     const int code = gcode[g];
     double4 xs;
     if (s < a.N) {
-        double4 vs = vel_o[s];
+        double4 vs = ldg_d4(vel_o + s);
         double fx, fy, fz;
         load_force<MIXED>(frc, frc32, s, fx, fy, fz);
         if (a.pre) kick(vs, fx, fy, fz, a.hp);
-        xs = integrate_one(pos_o[s], vs, fx, fy, fz, a.dt, a.h);
+        xs = integrate_one(ldg_d4(pos_o + s), vs, fx, fy, fz, a.dt, a.h);
     } else {
-        xs = pos_o[s];
+        xs = ldg_d4(pos_o + s);
     }
     const int base = GM == 1 ? 0 : 8;
     double4 x;
@@ -1272,16 +1272,16 @@ k_integrate(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, cons
     x.y = dadd(xs.y, dmul(a.len[1], (double)shift_axis(code, base, 1)));
     x.z = dadd(xs.z, dmul(a.len[2], (double)shift_axis(code, base, 2)));
     x.w = 0.0;
-    pos_n[t] = x;
+    st_d4(pos_n + t, x);
     if (MIXED) pos32_n[t] = rebased32(x, rbk[t], a.alo, a.rb_h);
     if (DEMV) {  // contact-fixed DEM: ghost velocity = its root's, after this half-kick
         const int r = groot[g];
-        double4 vr = vel_o[r];
+        double4 vr = ldg_d4(vel_o + r);
         double fx, fy, fz;
         load_force<MIXED>(frc, frc32, r, fx, fy, fz);
         if (a.pre) kick(vr, fx, fy, fz, a.hp);
         kick(vr, fx, fy, fz, a.h);
-        vel_n[t] = vr;
+        st_d4(vel_n + t, vr);
     }
 }
 
@@ -1295,7 +1295,7 @@ k_ghost_sync(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, con
     const int blk = (int)blockIdx.x + pdl_wait();
     const int t = blk * blockDim.x + threadIdx.x;
     if (t < a.N) {
-        pos_n[t] = pos_o[t];
+        st_d4(pos_n + t, ldg_d4(pos_o + t));
         if (MIXED) pos32_n[t] = pos32_o[t];
         return;
     }
@@ -1304,14 +1304,14 @@ k_ghost_sync(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, con
     const int s = GM == 1 ? gsrc[g] : groot[g];
     if (s < 0) return;  // received from another rank (halo exchange)
     const int code = gcode[g];
-    const double4 xs = pos_o[s];
+    const double4 xs = ldg_d4(pos_o + s);
     const int base = GM == 1 ? 0 : 8;
     double4 x;
     x.x = dadd(xs.x, dmul(a.len[0], (double)shift_axis(code, base, 0)));
     x.y = dadd(xs.y, dmul(a.len[1], (double)shift_axis(code, base, 1)));
     x.z = dadd(xs.z, dmul(a.len[2], (double)shift_axis(code, base, 2)));
     x.w = 0.0;
-    pos_n[t] = x;
+    st_d4(pos_n + t, x);
     if (MIXED) pos32_n[t] = rebased32(x, rbk[t], a.alo, a.rb_h);
     if (demv) vel[t] = vel[groot[g]];  // ghost slots only; roots are locals
 }
@@ -1330,21 +1330,21 @@ k_ghost_refresh(const double4* __restrict__ pos_o, double4* __restrict__ pos_n, 
     if (g >= a.G) return;
     const int t = a.N + g;
     if (GM == 0) {
-        pos_n[t] = pos_o[t];
+        st_d4(pos_n + t, ldg_d4(pos_o + t));
         if (MIXED) pos32_n[t] = pos32_o[t];
         return;
     }
     const int s = GM == 1 ? gsrc[g] : groot[g];
     if (s < 0) return;  // received from another rank (halo exchange)
     const int code = gcode[g];
-    const double4 xs = s < a.N ? pos_n[s] : pos_o[s];
+    const double4 xs = s < a.N ? pos_n[s] : ldg_d4(pos_o + s);
     const int base = GM == 1 ? 0 : 8;
     double4 x;
     x.x = dadd(xs.x, dmul(a.len[0], (double)shift_axis(code, base, 0)));
     x.y = dadd(xs.y, dmul(a.len[1], (double)shift_axis(code, base, 1)));
     x.z = dadd(xs.z, dmul(a.len[2], (double)shift_axis(code, base, 2)));
     x.w = 0.0;
-    pos_n[t] = x;
+    st_d4(pos_n + t, x);
     if (MIXED) pos32_n[t] = rebased32(x, rbk[t], a.alo, a.rb_h);
 }
 
@@ -1359,11 +1359,11 @@ k_final(double4* __restrict__ vel, const double4* __restrict__ frc, const float4
     if (i < N) {
         double fx, fy, fz;
         load_force<MIXED>(frc, frc32, i, fx, fy, fz);
-        double4 v = vel[i];
+        double4 v = ld_d4(vel + i);
         v.x = dadd(v.x, dmul(fx, h));
         v.y = dadd(v.y, dmul(fy, h));
         v.z = dadd(v.z, dmul(fz, h));
-        vel[i] = v;
+        st_d4(vel + i, v);
         if (THERMO) ke = v.x * v.x + v.y * v.y + v.z * v.z;
     }
     if (THERMO) put_partial(part, 3, ke, scratch);
@@ -1394,14 +1394,14 @@ __global__ void k_refresh_pos32(const double4* __restrict__ pos, float4* __restr
                                 const int* __restrict__ rbk, int NA, StepArgs a) {
     const int blk = (int)blockIdx.x + pdl_wait();
     const int t = blk * blockDim.x + threadIdx.x;
-    if (t < NA) pos32[t] = rebased32(pos[t], rbk[t], a.alo, a.rb_h);
+    if (t < NA) pos32[t] = rebased32(ldg_d4(pos + t), rbk[t], a.alo, a.rb_h);
 }
 
 __global__ void k_zero4(double4* __restrict__ d, float4* __restrict__ f, int n) {
     const int blk = (int)blockIdx.x + pdl_wait();
     const int t = blk * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    if (d) d[t] = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (d) st_d4(d + t, make_double4(0.0, 0.0, 0.0, 0.0));
     if (f) f[t] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
