@@ -23,6 +23,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <utility>
 #include <vector>
 
 #include "md_common.cuh"
@@ -71,7 +72,13 @@ double* gacc = nullptr;    // [3][nblk] per-block theta sums (eps, sigma, unused
 double* red = nullptr;     // [8] reduced sums
 int cap_n = 0, cap_seg = 0, cap_ck = 0;
 
-inline int nblk(int n) { return (n + kT - 1) / kT; }
+inline int nblk(long long n) { return (int)((n + kT - 1) / kT); }
+
+// Lanes per atom of the product kernel: more lanes shorten the chain of gathers and FP64 pair terms
+// that bounds a small system.  Kernel times in us by CUDA events (5 us of them the events), 4 / 8 / 16 /
+// 32 lanes: 864 atoms 16.7 / 12.7 / 10.8 / 9.0, 4,000 17.1 / 12.9 / 11.3 / 14.8, 8,788 17.0 / 14.5 / 16.9,
+// 16,384 19.0 / 21.1 / 23.1, 70,304 47.5 / 51.2 / 66.6.
+inline int hvp_lanes(int N) { return N <= 3000 ? 32 : N <= 6000 ? 16 : N <= 12000 ? 8 : 4; }
 
 struct HvpArgs {
     int N, stride, nbcap;
@@ -84,16 +91,16 @@ struct HvpArgs {
 
 // u_i = sum_j [f(s) w_ij + 2 f'(s) (d . w_ij) d],  w_ij = w_i - w_j, d = x_i - x_j,
 // f = 48 eps sr6 (sr6 - 1/2) sr2, f' = df/ds = 48 eps sr2^2 sr6 (2 - 7 sr6);
-// theta terms: w_i . F_i / eps and sum_j df/dsigma (d . w_i),
+// theta terms: sum_j f (d . w_i) / eps (= w_i . F_i / eps) and sum_j df/dsigma (d . w_i),
 // df/dsigma = (144 eps / sigma) sr2 sr6 (4 sr6 - 1).
-// The neighbour loop is split over kLpa adjacent lanes per atom (lane
+// The neighbour loop is split over kLpa adjacent lanes per atom (hvp_lanes; lane
 // `sub` takes entries sub, sub + kLpa, ...) in batches of kHb with the next batch's
 // entries loaded ahead, and the lanes' sums combined by shuffles.  Ghost neighbours
 // read their stored position (xs holds all slots of the step) and the adjoint of
 // their root through the root list `nbr`, so a neighbour costs two independent gathers.
-constexpr int kLpa = 4;  // lanes per atom
-constexpr int kHb = 2;   // neighbours per lane per batch
+constexpr int kHb = 2;  // neighbours per lane per batch (3 and 4: 110 registers, 47.5 -> 53.8 us at 70,304 atoms)
 
+template <int kLpa>
 __global__ void __launch_bounds__(kT)
 k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, double4* __restrict__ w_next,
                 double4* __restrict__ ax, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
@@ -103,7 +110,7 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
     const int t = blk * blockDim.x + threadIdx.x;
     const int i = t / kLpa, sub = t % kLpa;
     const bool act = i < a.N;
-    double ux = 0.0, uy = 0.0, uz = 0.0, Fx = 0.0, Fy = 0.0, Fz = 0.0, gs = 0.0;
+    double ux = 0.0, uy = 0.0, uz = 0.0, ge = 0.0, gs = 0.0;
     double4 wi = make_double4(0.0, 0.0, 0.0, 0.0);
     if (act) {
         const double4 xi = ldg_d4(xs + i);
@@ -141,14 +148,12 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
                     const double fp = 48.0 * a.eps * sr2 * sr2 * sr6 * (2.0 - 7.0 * sr6);
                     const double wx = wi.x - wj[b].x, wy = wi.y - wj[b].y, wz = wi.z - wj[b].z;
                     const double dw = 2.0 * fp * (dx * wx + dy * wy + dz * wz);
+                    const double di = dx * wi.x + dy * wi.y + dz * wi.z;
                     ux += f * wx + dw * dx;
                     uy += f * wy + dw * dy;
                     uz += f * wz + dw * dz;
-                    Fx += f * dx;
-                    Fy += f * dy;
-                    Fz += f * dz;
-                    gs += 144.0 * a.eps * a.inv_sigma * sr2 * sr6 * (4.0 * sr6 - 1.0) *
-                          (dx * wi.x + dy * wi.y + dz * wi.z);
+                    ge += f * di;
+                    gs += 144.0 * a.eps * a.inv_sigma * sr2 * sr6 * (4.0 * sr6 - 1.0) * di;
                 }
             }
         }
@@ -158,13 +163,9 @@ k_adj_hvp_split(const double4* __restrict__ xs, const double4* __restrict__ w, d
         ux += __shfl_xor_sync(0xffffffffu, ux, o);
         uy += __shfl_xor_sync(0xffffffffu, uy, o);
         uz += __shfl_xor_sync(0xffffffffu, uz, o);
-        Fx += __shfl_xor_sync(0xffffffffu, Fx, o);
-        Fy += __shfl_xor_sync(0xffffffffu, Fy, o);
-        Fz += __shfl_xor_sync(0xffffffffu, Fz, o);
     }
-    double ge = 0.0;
+    ge /= a.eps;
     if (act && sub == 0) {
-        ge = (wi.x * Fx + wi.y * Fy + wi.z * Fz) / a.eps;
         double4 q = ld_d4(ax + i);
         q.x += a.kick * ux;
         q.y += a.kick * uy;
@@ -376,17 +377,41 @@ void checkpoint(State& s, int k) {
     launched(K_ADJ_STEP);
 }
 
-// one forward step t (positions x_t -> x_{t+1}); reneighbours when (t+1) % R == 0
-void forward_step(State& s, int t, bool allow_reneigh) {
-    const bool ren = allow_reneigh && (t + 1) % cfg.reneigh == 0;
-    if (ren) {
-        run_integrate(s, cfg.dt, false);
+// the ghosts and lists after an integration to x_{t+1}: rebuilt when (t+1) % R == 0, else the ghosts
+// refreshed where the integrating kernel has not written them
+void finish_move(State& s, int t, bool pushed) {
+    if ((t + 1) % cfg.reneigh == 0) {
         run_enforce_pbc(s);
         rebuild(s);
-    } else {
-        run_integrate(s, cfg.dt, true);
+    } else if (!pushed && s.ghosts_pushed != 2) {
+        run_ghost_refresh(s, 2);
     }
-    run_force_lj(s, force_params(), true, cfg.dt);
+}
+
+// The velocity-Verlet steps t0 .. t1-1 from x_t0 (with its force) on: one kernel per step, the force at
+// x_{t+1}, its kick and the integration to x_{t+2}, as the driver's loop runs it; after_step(t) is called
+// with x_{t+1}, v_{t+1} in place wherever stop(t) asks for it, and after the last step.  move(t) is
+// called before the launch that writes x_{t+1}.
+template <class Stop, class After, class Move>
+void run_steps(State& s, int t0, int t1, bool last_force, Stop stop, After after_step, Move move) {
+    bool moved = false;  // x_{t+1} is there already
+    for (int t = t0; t < t1; ++t) {
+        if (!moved) {
+            move(t);
+            const bool ren = (t + 1) % cfg.reneigh == 0;
+            run_integrate(s, cfg.dt, !ren);
+            finish_move(s, t, true);
+        }
+        moved = t + 1 < t1 && !stop(t);
+        if (moved) {
+            move(t + 1);
+            run_force_lj_init(s, force_params(), cfg.dt, cfg.dt);
+            finish_move(s, t + 1, false);
+        } else if (t + 1 < t1 || last_force) {
+            run_force_lj(s, force_params(), true, cfg.dt);
+            after_step(t);
+        }
+    }
 }
 
 struct ModeGuard {  // the adjoint runs exact ghosts, full lists, its own precision, no thermo
@@ -456,6 +481,16 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     dalloc(&x0_dev, N);
     dfree(&mass_ref);
     dalloc(&mass_ref, N);
+    // the reverse pass's buffers too, so that nothing waits for the device behind the steps
+    const int nbs = nblk((long long)hvp_lanes(N) * N);  // blocks of its product kernel
+    for (double4** p : {&ax, &av[0], &av[1], &tmp4}) {
+        dfree(p);
+        dalloc(p, N);
+    }
+    dfree(&gacc);
+    dalloc(&gacc, 2 * (size_t)nbs + 2);
+    dfree(&red);
+    dalloc(&red, 8);
     // initial state in reference order: x_0 from md_initialize_grid, v_0 from the caller
     materialize_mirror(s);
     const double* x0 = s.x0_in_pos ? s.h_pos.data() : s.h_x0.data();
@@ -478,26 +513,16 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     reset_identity(s, 0);
     rebuild(s);
     run_force_lj(s, force_params(), false, 0.0);
-    for (int t = 0; t < cfg.steps; ++t) {
-        forward_step(s, t, true);
-        if ((t + 1) % cfg.reneigh == 0 && t + 1 < cfg.steps) checkpoint(s, (t + 1) / cfg.reneigh);
-    }
+    auto checkpoint_after = [&](int t) { return (t + 1) % cfg.reneigh == 0 && t + 1 < cfg.steps; };
+    run_steps(
+        s, 0, cfg.steps, true, checkpoint_after,
+        [&](int t) {
+            if (checkpoint_after(t)) checkpoint(s, (t + 1) / cfg.reneigh);
+        },
+        [](int) {});
     cudaEventRecord(e1, s.stream);
     // loss: MSD and U at x_T, and the initial adjoint state
     const int nb = nblk(N);
-    dfree(&ax);
-    dalloc(&ax, N);
-    dfree(&av[0]);
-    dfree(&av[1]);
-    dalloc(&av[0], N);
-    dalloc(&av[1], N);
-    dfree(&tmp4);
-    dalloc(&tmp4, N);
-    dfree(&gacc);
-    const int nbs = nblk(kLpa * N);  // blocks of the reverse pass's product kernel
-    dalloc(&gacc, 2 * (size_t)nbs + 2);
-    dfree(&red);
-    dalloc(&red, 8);
     flush_thermo(s);  // sums of a forward run waiting in the scratch
     ensure_red_scratch(s, 8 * nb);
     const double sig6 = std::pow(sigma, 6);
@@ -535,10 +560,10 @@ int md_adjoint_forward(double const* v0, double epsilon, double sigma, double* l
     // adjoint state to reference order (the backward pass starts in another layout)
     launch(s, nb, kT, 0, k_to_ref, ax, s.ref.b[s.ac], tmp4, N);
     launched(K_ADJ_STEP);
-    TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+    std::swap(ax, tmp4);
     launch(s, nb, kT, 0, k_to_ref, av[0], s.ref.b[s.ac], tmp4, N);
     launched(K_ADJ_STEP);
-    TMD_CUDA(cudaMemcpyAsync(av[0], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+    std::swap(av[0], tmp4);
     TMD_CUDA(cudaStreamSynchronize(s.stream));
     guard.restore(s);
     *loss = run.loss;
@@ -554,7 +579,8 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
     }
     const int N = s.N;
     const int nb = nblk(N);
-    const int nbs = nblk(kLpa * N);
+    const int lanes = hvp_lanes(N);
+    const int nbs = nblk((long long)lanes * N);
     const int R = cfg.reneigh;
     ModeGuard guard(s);
     cudaEvent_t e0, e1;
@@ -563,6 +589,7 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
     cudaEventRecord(e0, s.stream);
     const double c = 0.5 * cfg.dt;
     int wcur = 0;  // av[wcur] holds a_v (reference order between segments)
+    std::vector<const double4*> x_at;  // a segment's positions, step by step
     for (int seg = run.nseg - 1; seg >= 0; --seg) {
         const int t0 = seg * R;
         const int t1 = std::min(t0 + R, cfg.steps);  // positions x_t0 .. x_{t1-1}
@@ -584,20 +611,27 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
         launch(s, nb, kT, 0, k_root_list, s.nbn, s.nbl, s.groot, nbr, N, s.nb_stride, s.nb_cap);
         launched(K_ADJ_STEP);
         run_force_lj(s, force_params(), false, 0.0);
-        TMD_CUDA(cudaMemcpyAsync(seg_x, s.pos.b[s.pc], sizeof(double4) * NA, cudaMemcpyDeviceToDevice, s.stream));
-        for (int t = t0; t + 1 < t1; ++t) {
-            forward_step(s, t, false);
-            TMD_CUDA(cudaMemcpyAsync(seg_x + (size_t)(t + 1 - t0) * NA, s.pos.b[s.pc], sizeof(double4) * NA,
-                                     cudaMemcpyDeviceToDevice, s.stream));
-        }
+        // x_t0 stays in the position buffer; each later step writes its positions straight into its
+        // own part of seg_x, which stands in for the buffer written
+        double4* const own[2] = {s.pos.b[0], s.pos.b[1]};
+        x_at.assign(1, s.pos.b[s.pc]);
+        run_steps(
+            s, t0, t1 - 1, seg == 0, [](int) { return false; }, [](int) {},
+            [&](int t) {
+                double4* next = seg_x + (size_t)(t + 1 - t0) * NA;
+                s.pos.b[1 - s.pc] = next;
+                x_at.push_back(next);
+            });
+        s.pos.b[0] = own[0];
+        s.pos.b[1] = own[1];
         // adjoint state into this segment's slot order
         const int* ref = s.ref.b[s.ac];
         launch(s, nb, kT, 0, k_from_ref, ax, ref, tmp4, N);
         launched(K_ADJ_STEP);
-        TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+        std::swap(ax, tmp4);
         launch(s, nb, kT, 0, k_from_ref, av[wcur], ref, tmp4, N);
         launched(K_ADJ_STEP);
-        TMD_CUDA(cudaMemcpyAsync(av[wcur], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+        std::swap(av[wcur], tmp4);
         HvpArgs a;
         a.N = N;
         a.stride = s.nb_stride;
@@ -612,18 +646,26 @@ int md_adjoint_backward(double* grad_v0, double* grad_eps, double* grad_sigma) {
             a.drift = t > 0 ? cfg.dt : 0.0;
             a.wt = t > 0 ? cfg.dt : c;
             prof_begin(K_HVP);
-            launch(s, nbs, kT, 0, k_adj_hvp_split, seg_x + (size_t)(t - t0) * NA, av[wcur], av[1 - wcur], ax, s.nbn,
-                   s.nbl, nbr, gacc, a);
+            auto product = [&](auto kernel) {
+                launch(s, nbs, kT, 0, kernel, x_at[t - t0], av[wcur], av[1 - wcur], ax, s.nbn, s.nbl, nbr, gacc, a);
+            };
+            if (lanes == 32) product(k_adj_hvp_split<32>);
+            else if (lanes == 16) product(k_adj_hvp_split<16>);
+            else if (lanes == 8) product(k_adj_hvp_split<8>);
+            else product(k_adj_hvp_split<4>);
             launched(K_HVP);
             prof_end(K_HVP);
             wcur = 1 - wcur;
         }
+        if (seg == 0 && x_at.size() > 1)  // the grid is left at the last recomputed positions, in its own buffer
+            TMD_CUDA(cudaMemcpyAsync(s.pos.b[s.pc], x_at.back(), sizeof(double4) * NA, cudaMemcpyDeviceToDevice,
+                                     s.stream));
         launch(s, nb, kT, 0, k_to_ref, ax, ref, tmp4, N);
         launched(K_ADJ_STEP);
-        TMD_CUDA(cudaMemcpyAsync(ax, tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+        std::swap(ax, tmp4);
         launch(s, nb, kT, 0, k_to_ref, av[wcur], ref, tmp4, N);
         launched(K_ADJ_STEP);
-        TMD_CUDA(cudaMemcpyAsync(av[wcur], tmp4, sizeof(double4) * N, cudaMemcpyDeviceToDevice, s.stream));
+        std::swap(av[wcur], tmp4);
     }
     cudaEventRecord(e1, s.stream);
     // theta gradients: per-block sums plus the direct terms stored after them
