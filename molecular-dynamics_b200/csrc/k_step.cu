@@ -649,7 +649,13 @@ __device__ __forceinline__ void push_chain_block(int block, const double4* __res
         push_chain<MIXED>(q, pos, N, pa, pos_n, pos32_n, alo, rb_h);
 }
 
-// The pair arithmetic and the FP64-path queue of k_lj_mixed_bf; the lanes' sums are added in FP64.
+// Mixed: the pair arithmetic of k_lj_mixed_bf, bit for bit.  A round takes 4 L list entries (a quad per
+// lane); the lanes put each pair's del and f into shared memory, and the atom's lanes add the
+// components in list order with the same fused multiply-adds (a pair in no window has f = 0).  The
+// quads with FP64-path pairs are marked and worked off after the rounds, in list order, by all lanes of
+// the atom alike.  Adding each lane's own sum instead took 7.5, 11.9 and 14.8 us a step at 2,048, 16,384
+// and 29,716 atoms against 8.9, 14.0 and 19.4, but then a trajectory leaves the thread-per-atom
+// kernel's by roundings, which a hundred chaotic steps turn into other cutoff crossings.
 template <int L, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
 __global__ void __launch_bounds__(kThreads)
 k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ pos, float4* __restrict__ frc32,
@@ -658,69 +664,133 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
                  float4* __restrict__ pos32_n = nullptr, const int* __restrict__ rbk = nullptr,
                  PushArgs pa = PushArgs()) {
     const int blk = (int)blockIdx.x + pdl_wait();
+    static_assert(L >= 4 && L <= 32, "three lanes of an atom add its force's components");
+    constexpr int kAtoms = 32 / L;    // atoms per warp
+    constexpr int kRow = 4 * L + 4;   // a round of one of dx, dy, dz, f: strides that keep the 16-byte
+    constexpr int kAtom = 4 * kRow;   // accesses of eight lanes on different banks
+    constexpr int kMarks = 64;        // quads with a mark of FP64-path pairs; a longer list is tested again
     __shared__ double scratch[kThreads / 32];
-    __shared__ int s_q[kQQ + 1][kThreads];
+    __shared__ __align__(16) float s_p[kThreads / 32][kAtoms * kAtom];
+    __shared__ unsigned char s_slow[kThreads / 32][kAtoms][kMarks];
     if (INIT && lists_failed(a)) return;  // the whole grid returns: nothing written
     double e = 0.0, w = 0.0, cnt = 0.0, ke = 0.0;
     if (blk < atom_blocks) {
+        const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int t = blk * kThreads + threadIdx.x;
-        const int i = t / L, sub = t % L;
+        const int i = t / L, sub = t % L, at = lane / L;
         const bool act = i < a.N;
         const int n = act ? min(nbn[i], a.nbcap) : 0;
         const float4 ri = act ? pos32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        float fx = 0.f, fy = 0.f, fz = 0.f, ef = 0.f, wf = 0.f;
-        double cx = 0.0, cy = 0.0, cz = 0.0;
-        int ncnt = 0, nq = 0;
+        float ef = 0.f, wf = 0.f, none[3] = {0.f, 0.f, 0.f};
+        int ncnt = 0;
+        float acc = 0.f;  // component `sub` of the force (sub < 3)
+        unsigned long long marks = 0;  // the atom's quads with FP64-path pairs, below kMarks
+        bool more = false;             // some beyond
         const int nquad = (n + 3) >> 2;
-        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
-        for (int b = sub; b < nquad; b += L) {
+        const int rounds = __reduce_max_sync(0xffffffffu, (nquad + L - 1) / L);
+        // the next round's gathers are in flight while this one's forces are added, and the quad of the
+        // round after that
+        const uint4 empty = make_uint4(0u, 0u, 0u, 0u);
+        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : empty;
+        uint4 en = sub + L < nquad ? list_quad(nbl, sub + L, i, a.stride) : empty;
+        float4 rj[kB32];
+        auto gather = [&](const uint4& q) {
+            rj[0] = __ldg(pos32 + (q.x >> kCodeBits));
+            rj[1] = __ldg(pos32 + (q.y >> kCodeBits));
+            rj[2] = __ldg(pos32 + (q.z >> kCodeBits));
+            rj[3] = __ldg(pos32 + (q.w >> kCodeBits));
+        };
+        gather(eq);
+        float* const row = s_p[wid] + at * kAtom;
+        for (int r = 0; r < rounds; ++r) {
+            const int b = r * L + sub;
             const uint32_t cur[kB32] = {eq.x, eq.y, eq.z, eq.w};
-            float4 rj[kB32];
-#pragma unroll
-            for (int u = 0; u < kB32; ++u) rj[u] = __ldg(pos32 + (cur[u] >> kCodeBits));
-            if (b + L < nquad) eq = list_quad(nbl, b + L, i, a.stride);
             unsigned slow = 0;
+            float d[4][kB32];
 #pragma unroll
-            for (int u = 0; u < kB32; ++u)
-                slow |= mixed_pair<THERMO>(cur[u], ri, rj[u], a, fx, fy, fz, ef, wf, ncnt) ? (1u << u) : 0u;
-            s_q[min(nq, kQQ)][threadIdx.x] = (b << kB32) | (int)slow;
-            nq += slow != 0u ? 1 : 0;
-        }
-        if (nq > kQQ) {  // more than the queue holds: this lane's quads again, FP64 pairs in place
-            fx = fy = fz = ef = wf = 0.f;
-            ncnt = 0;
-            const double4 pi = ldg_d4(pos + i);
-            for (int b = sub; b < nquad; b += L) {
-                const uint4 e4 = list_quad(nbl, b, i, a.stride);
-                const uint32_t c4[kB32] = {e4.x, e4.y, e4.z, e4.w};
-                for (int u = 0; u < kB32; ++u) {
-                    const int j = (int)(c4[u] >> kCodeBits);
-                    if (mixed_pair<THERMO>(c4[u], ri, __ldg(pos32 + j), a, fx, fy, fz, ef, wf, ncnt))
-                        fp64_lj<THERMO>(pi, j, pos, a, cx, cy, cz, e, w, ncnt);
+            for (int u = 0; u < kB32; ++u) {
+                const float rsq = mixed_del(cur[u], ri, rj[u], a, d[0][u], d[1][u], d[2][u]);
+                const bool fast = mixed_fast(rsq, a);
+                float sr2, t6;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(sr2) : "f"(rsq));
+                float f = mixed_force(sr2, a, t6);
+                const bool on = b < nquad;
+                f = fast && on ? f : 0.f;
+                d[3][u] = f;
+                if (THERMO) {
+                    ef += fast && on ? t6 * fmaf(a.lj_c, t6, a.lj_d) : 0.f;
+                    wf = on ? fmaf(f, rsq, wf) : wf;
+                    ncnt += fast && on ? 1 : 0;
+                }
+                slow |= on && !fast && rsq < a.rc2_hi ? (1u << u) : 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<float4*>(row + c * kRow + 4 * sub) = make_float4(d[c][0], d[c][1], d[c][2], d[c][3]);
+            eq = en;
+            gather(eq);
+            en = b + 2 * L < nquad ? list_quad(nbl, b + 2 * L, i, a.stride) : empty;
+            if (slow != 0u && b < kMarks) s_slow[wid][at][b] = (unsigned char)slow;
+            const unsigned any = __ballot_sync(0xffffffffu, slow != 0u) >> (lane & ~(L - 1)) & ((1ull << L) - 1ull);
+            if (r * L < kMarks) marks |= (unsigned long long)any << (r * L);
+            more = more || (any != 0u && (r + 1) * L > kMarks);
+            __syncwarp();
+            if (sub < 3) {
+                const float* q = row + sub * kRow;
+#pragma unroll
+                for (int k = 0; k < L; ++k) {
+                    const float4 v = *reinterpret_cast<const float4*>(q + 4 * k);
+                    const float4 f = *reinterpret_cast<const float4*>(row + 3 * kRow + 4 * k);
+                    acc = fmaf(v.x, f.x, acc);
+                    acc = fmaf(v.y, f.y, acc);
+                    acc = fmaf(v.z, f.z, acc);
+                    acc = fmaf(v.w, f.w, acc);
                 }
             }
-        } else if (nq > 0) {
+            __syncwarp();
+        }
+        const int base = lane & ~(L - 1);
+        const float fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
+                    fz = __shfl_sync(0xffffffffu, acc, base + 2);
+        // the FP64 pairs of the atom, in list order; every lane of it runs them (THERMO: lane 0 counts)
+        double cx = 0.0, cy = 0.0, cz = 0.0, e64 = 0.0, w64 = 0.0;
+        int n64 = 0;
+        if (marks != 0 || more) {
             const double4 pi = ldg_d4(pos + i);
-            for (int q = 0; q < nq; ++q) {
-                const int wq = s_q[q][threadIdx.x];
-                const uint4 e4 = list_quad(nbl, wq >> kB32, i, a.stride);
-                unsigned bits = (unsigned)wq & ((1u << kB32) - 1u);
+            auto run = [&](const uint4& e4, unsigned bits) {
                 while (bits) {
                     const int u = __ffs(bits) - 1;
                     bits &= bits - 1u;
                     const uint32_t en = u == 0 ? e4.x : (u == 1 ? e4.y : (u == 2 ? e4.z : e4.w));
-                    fp64_lj<THERMO>(pi, (int)(en >> kCodeBits), pos, a, cx, cy, cz, e, w, ncnt);
+                    fp64_lj<THERMO>(pi, (int)(en >> kCodeBits), pos, a, cx, cy, cz, e64, w64, n64);
                 }
+            };
+            while (marks) {
+                const int b = __ffsll(marks) - 1;
+                marks &= marks - 1ull;
+                run(list_quad(nbl, b, i, a.stride), s_slow[wid][at][b]);
+            }
+            for (int b = kMarks; more && b < nquad; ++b) {
+                const uint4 e4 = list_quad(nbl, b, i, a.stride);
+                const uint32_t c4[kB32] = {e4.x, e4.y, e4.z, e4.w};
+                unsigned bits = 0;
+                float unused = 0.f;
+                int unused_n = 0;
+                for (int u = 0; u < kB32; ++u)
+                    bits |= mixed_pair<false>(c4[u], ri, __ldg(pos32 + (c4[u] >> kCodeBits)), a, none[0], none[1],
+                                              none[2], unused, unused, unused_n)
+                                ? (1u << u)
+                                : 0u;
+                run(e4, bits);
             }
         }
-        double Fx = (double)fx + cx, Fy = (double)fy + cy, Fz = (double)fz + cz;
         __syncwarp();
-#pragma unroll
-        for (int o = 1; o < L; o <<= 1) {
-            Fx += __shfl_xor_sync(0xffffffffu, Fx, o);
-            Fy += __shfl_xor_sync(0xffffffffu, Fy, o);
-            Fz += __shfl_xor_sync(0xffffffffu, Fz, o);
+        if (THERMO && sub == 0) {
+            e = e64;
+            w = w64;
+            ncnt += n64;
         }
+        const double Fx = (double)fx + cx, Fy = (double)fy + cy, Fz = (double)fz + cz;
         const float4 F = make_float4((float)Fx, (float)Fy, (float)Fz, 0.f);
         if (act && sub == 0) frc32[i] = F;
         if (FUSE) {
@@ -771,7 +841,7 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
     static_assert(L >= 4 && L <= 32, "three lanes of an atom add its force's components");
     // pairs outside the cutoff evaluated too, without a branch: shorter chains (2,048 atoms, 8 lanes:
     // step 12.9 -> 12.2 us) but more work (16,384 atoms, 4 lanes: 18.1 -> 19.2 us)
-    constexpr bool kFlat = L >= 8;
+    constexpr bool kFlat = L >= 8, kAhead = L >= 8;
     constexpr int kAtoms = 32 / L;       // atoms per warp
     // a component's 4 L doubles of a round, and an atom's three components: strides that keep the
     // 16-byte writes of eight lanes and the reads of an atom's three on different banks
@@ -791,14 +861,26 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
         double acc = 0.0;  // component `sub` of the force (sub < 3)
         const int nquad = (n + 3) >> 2;
         const int rounds = __reduce_max_sync(0xffffffffu, (nquad + L - 1) / L);
-        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        // kAhead: the next round's gathers are in flight while this one's forces are added, and the quad
+        // of the round after that
+        const uint4 empty = make_uint4(0u, 0u, 0u, 0u);
+        uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : empty;
+        uint4 en = sub + L < nquad ? list_quad(nbl, sub + L, i, a.stride) : empty;
+        double4 pj[kB64];
+        auto gather = [&](const uint4& q) {
+            pj[0] = ldg_d4(pos + (q.x >> kCodeBits));
+            pj[1] = ldg_d4(pos + (q.y >> kCodeBits));
+            pj[2] = ldg_d4(pos + (q.z >> kCodeBits));
+            pj[3] = ldg_d4(pos + (q.w >> kCodeBits));
+        };
+        if (kAhead) gather(eq);
         for (int r = 0; r < rounds; ++r) {
             const int b = r * L + sub;
-            const uint32_t ent[kB64] = {eq.x, eq.y, eq.z, eq.w};
-            double4 pj[kB64];
-#pragma unroll
-            for (int u = 0; u < kB64; ++u) pj[u] = ldg_d4(pos + (ent[u] >> kCodeBits));
-            if (b + L < nquad) eq = list_quad(nbl, b + L, i, a.stride);
+            if (!kAhead) {
+                gather(eq);
+                eq = en;
+                en = b + 2 * L < nquad ? list_quad(nbl, b + 2 * L, i, a.stride) : empty;
+            }
             double p[3][kB64];
 #pragma unroll
             for (int u = 0; u < kB64; ++u) {
@@ -828,6 +910,11 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
                 for (int h = 0; h < 2; ++h)
                     *reinterpret_cast<double2*>(row + c * kRow + h * 2 * L + 2 * sub) =
                         make_double2(p[c][2 * h], p[c][2 * h + 1]);
+            if (kAhead) {
+                eq = en;
+                gather(eq);
+                en = b + 2 * L < nquad ? list_quad(nbl, b + 2 * L, i, a.stride) : empty;
+            }
             __syncwarp();
             if (sub < 3) {
                 const double* q = row + sub * kRow;
@@ -1160,43 +1247,62 @@ k_dem_mixed(const float4* __restrict__ pos32, const double4* __restrict__ pos, c
     }
 }
 
-// few grains, L lanes to a grain (see k_dem_fp64_lanes); the lanes' sums are added in FP64
+// few grains, L lanes to a grain (see k_dem_fp64_lanes): the FP32 forces and the FP64 ones of pairs near
+// a decision are added in list order, k_dem_mixed's bits
 template <int L>
 __global__ void __launch_bounds__(kThreads)
 k_dem_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ pos, const double4* __restrict__ vel,
                   float4* __restrict__ frc32, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, DemArgs a,
                   DemMixedArgs b) {
+    static_assert(L >= 4, "three lanes of a grain add its force's components");
     const int blk = (int)blockIdx.x + pdl_wait();
+    __shared__ float s_f[3][kThreads + 4];
+    __shared__ double s_c[3][kThreads + 4];
     const int t = blk * kThreads + threadIdx.x;
     const int i = t / L, sub = t % L;
-    float f[3] = {0.f, 0.f, 0.f};
-    double c[3] = {0.0, 0.0, 0.0};
-    if (i < a.N && a.fixed) {
-        const float4 ri = pos32[i];
-        const double4 v = ldg_d4(vel + i);
-        const float3 vi = make_float3((float)v.x, (float)v.y, (float)v.z);
-        const int n = min(nbn[i], a.nbcap);
-        uint32_t en = sub < n ? __ldg(nbl + nl_index(sub, i, a.stride)) : 0u;
-        float4 rn = __ldg(pos32 + (en >> kCodeBits));
-        for (int k = sub; k < n; k += L) {
-            const uint32_t e0 = en;
-            const float4 rj = rn;
-            if (k + L < n) {
-                en = __ldg(nbl + nl_index(k + L, i, a.stride));
-                rn = __ldg(pos32 + (en >> kCodeBits));
-            }
-            dem_mixed_pair<false>(e0, i, ri, rj, v, vi, pos, vel, frc32, nullptr, a, b, f, c);
+    const int ic = i < a.N ? i : 0;
+    const int n = i < a.N && a.fixed ? min(nbn[i], a.nbcap) : 0;
+    const int rounds = __reduce_max_sync(0xffffffffu, (n + L - 1) / L);
+    const float4 ri = pos32[ic];
+    const double4 v = ldg_d4(vel + ic);
+    const float3 vi = make_float3((float)v.x, (float)v.y, (float)v.z);
+    float accf = 0.f;  // component `sub` of the force (sub < 3)
+    double accc = 0.0;
+    uint32_t en = sub < n ? __ldg(nbl + nl_index(sub, ic, a.stride)) : 0u;
+    float4 rn = __ldg(pos32 + (en >> kCodeBits));
+    for (int r = 0; r < rounds; ++r) {
+        const int k = r * L + sub;
+        const uint32_t e0 = en;
+        const float4 rj = rn;
+        if (k + L < n) {
+            en = __ldg(nbl + nl_index(k + L, ic, a.stride));
+            rn = __ldg(pos32 + (en >> kCodeBits));
         }
+        float f[3] = {0.f, 0.f, 0.f};
+        double c[3] = {0.0, 0.0, 0.0};
+        if (k < n) dem_mixed_pair<false>(e0, ic, ri, rj, v, vi, pos, vel, frc32, nullptr, a, b, f, c);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            s_f[d][threadIdx.x] = f[d];
+            s_c[d][threadIdx.x] = c[d];
+        }
+        __syncwarp();
+        if (sub < 3) {
+            const float* q = s_f[sub] + (threadIdx.x - sub);
+            const double* p = s_c[sub] + (threadIdx.x - sub);
+#pragma unroll
+            for (int m = 0; m < L; ++m) {
+                accf += q[m];
+                accc += p[m];
+            }
+        }
+        __syncwarp();
     }
-    double F[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) F[d] = (double)f[d] + c[d];
-    __syncwarp();
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) F[d] += __shfl_xor_sync(0xffffffffu, F[d], o);
-    if (i < a.N && sub == 0) frc32[i] = make_float4((float)F[0], (float)F[1], (float)F[2], 0.f);
+    const float F = (float)((double)accf + accc);
+    const int base = (threadIdx.x & 31) - sub;
+    const float fx = __shfl_sync(0xffffffffu, F, base), fy = __shfl_sync(0xffffffffu, F, base + 1),
+                fz = __shfl_sync(0xffffffffu, F, base + 2);
+    if (i < a.N && sub == 0) frc32[i] = make_float4(fx, fy, fz, 0.f);
 }
 
 // ---- integration + ghost refresh ------------------------------------------------
@@ -1437,16 +1543,17 @@ StepArgs step_args(const State& s, double dt) {
 
 // Lanes per atom of a full-list LJ force kernel (1: the thread-per-atom kernels).  More lanes
 // shorten the chain of gathers that bounds a small system; a system that fills the chip pays for
-// them (the sums across lanes, the FP64 form's exchange through shared memory).  Step times in us
-// (LJ liquid, rebuild every 20 steps included), 1 / 2 / 4 / 8 / 16 lanes:
-//   mixed  2,048 atoms 21 / 15.7 / 13.0 / 11.6 / 11.0    16,384  22 / 17.7 / 15.7 / 15.8 / 19.7
-//         42,592       25 / 21.6 / 20.4 / 26.5 / 31      70,304  28.6 / 26.4 / 30.1   87,808 33.3 / 33.6 / 35.8
-//   FP64   2,048 atoms 25.3 / - / 14.9 / 11.9 / 11.8      5,148  26.8 / - / 15.0 / 13.1 / 15.0
-//          7,488       25.6 / - / 15.0 / 15.0 / 17.0     32,000  28.2 / - / 24.3 / 32.5   42,592 29.1 / - / 35.8
+// adding the pair forces in list order across them.  Step times in us (LJ liquid, rebuild every 20
+// steps included), 1 / 4 / 8 / 16 lanes:
+//   mixed  256 atoms 15.6 /  9.2 /  8.3 /  8.0    2,048 16.6 / 10.3 /  8.9 /  9.0    5,148 18.0 / 10.9 / 10.4 / 11.3
+//         10,976     17.9 / 12.8 / 13.1 / 18.3   16,384 17.7 / 14.0 / 15.7 / 21.5   29,716 20.0 / 19.4 / 25.6
+//         55,296     22.7 / 32.9 (2 lanes: 29,716 19.2, 55,296 25.7)
+//   FP64   256 atoms 19.2 /  9.6 /  7.4 /  6.8    2,048 21.4 / 10.2 /  7.8 /  7.8    5,148 22.3 / 10.8 /  9.8 / 10.7
+//         10,976     22.4 / 12.3 / 13.1 / 18.0   29,716 24.2 / 20.7 / 27.6           42,592 25.2 / 30.7
 int force_lanes(int N, bool mixed) {
-    if (N <= 2048) return 16;
-    if (mixed) return N <= 16384 ? 8 : N <= 49152 ? 4 : N <= 81920 ? 2 : 1;
-    return N <= 7168 ? 8 : N <= 38912 ? 4 : 1;
+    if (N <= (mixed ? 1024 : 2048)) return 16;
+    if (N <= 8192) return 8;
+    return N <= (mixed ? 29000 : 36000) ? 4 : 1;
 }
 
 // blocks of a full-list LJ force launch over N atoms and nchain chain ghosts
@@ -1456,18 +1563,16 @@ int force_blocks(int N, int lanes, int nchain) {
 }
 
 template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
-void launch_lj_mixed_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
-    launch(s, nb, kThreads, 0, (k_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos32.b[s.pc], s.pos.b[s.pc],
-           s.frc32, s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a, nblocks((long long)a.N * L, kThreads),
-           INIT ? s.pos.b[1 - s.pc] : nullptr, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
-}
-
-template <int L, bool FUSE, bool THERMO, bool INIT, bool PUSH>
 void launch_lj_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
-    if (s.precision == 1) return launch_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
-    launch(s, nb, kThreads, 0, (k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac],
-           s.vel.b[s.vc], s.nbn, s.nbl, s.red_part, a, nblocks((long long)a.N * L, kThreads),
-           INIT ? s.pos.b[1 - s.pc] : nullptr, pa);
+    double4* vel = s.vel.b[s.vc];
+    double4* pn = INIT ? s.pos.b[1 - s.pc] : nullptr;
+    const int ab = nblocks((long long)a.N * L, kThreads);
+    if (s.precision == 1)
+        launch(s, nb, kThreads, 0, (k_lj_mixed_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos32.b[s.pc], s.pos.b[s.pc],
+               s.frc32, vel, s.nbn, s.nbl, s.red_part, a, ab, pn, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
+    else
+        launch(s, nb, kThreads, 0, (k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac], vel,
+               s.nbn, s.nbl, s.red_part, a, ab, pn, pa);
 }
 
 // INIT: the kernels write the integrated locals into the other position buffer
@@ -1477,9 +1582,6 @@ void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs&
     double4* pn = INIT ? s.pos.b[1 - s.pc] : nullptr;
     if constexpr (!HALF) {
         switch (lanes) {
-            case 2:  // the mixed form only
-                if (s.precision == 1) return launch_lj_mixed_lanes<2, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
-                break;
             case 4: return launch_lj_lanes<4, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
             case 8: return launch_lj_lanes<8, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
             case 16: return launch_lj_lanes<16, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
