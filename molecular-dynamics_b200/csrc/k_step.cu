@@ -179,7 +179,9 @@ __device__ __forceinline__ void push_chain(int q, const double4* __restrict__ po
 // INIT (with FUSE, full lists): the epilogue also does the next step's initial integration
 // and writes the atom's new position to pos_n, the other buffer (neighbours read pos)
 // PUSH (with INIT): the kernel also writes the ghosts (PushArgs)
-template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
+// AHEAD: the next quad's gathers are in flight while this one's pairs run; its registers leave five
+// blocks per SM instead of eight (force_ahead chooses)
+template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false>
 __global__ void __launch_bounds__(kThreads)
 k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
           const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot,
@@ -200,16 +202,32 @@ k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* _
         // (entries past n are padding, skipped below)
         const int nq = (n + 3) >> 2;
         uint4 eq = n > 0 ? list_quad(nbl, 0, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        uint4 en = AHEAD && nq > 1 ? list_quad(nbl, 1, i, a.stride) : eq;
+        double4 pn[kB64];
+        auto gather = [&](const uint4& q) {
+            pn[0] = ldg_d4(pos + (q.x >> kCodeBits));
+            pn[1] = ldg_d4(pos + (q.y >> kCodeBits));
+            pn[2] = ldg_d4(pos + (q.z >> kCodeBits));
+            pn[3] = ldg_d4(pos + (q.w >> kCodeBits));
+        };
+        if (AHEAD) gather(eq);
         for (int b = 0; b < nq; ++b) {
             const int k0 = 4 * b;
             const uint32_t ent[kB64] = {eq.x, eq.y, eq.z, eq.w};
             int j[kB64];
-            double4 pj[kB64];
 #pragma unroll
             for (int u = 0; u < kB64; ++u) j[u] = (int)(ent[u] >> kCodeBits);
+            double4 pj[kB64];
+            if (!AHEAD) gather(eq);
 #pragma unroll
-            for (int u = 0; u < kB64; ++u) pj[u] = ldg_d4(pos + j[u]);
-            eq = list_quad(nbl, min(b + 1, nq - 1), i, a.stride);
+            for (int u = 0; u < kB64; ++u) pj[u] = pn[u];
+            if (AHEAD) {
+                eq = en;
+                gather(eq);
+                en = list_quad(nbl, min(b + 2, nq - 1), i, a.stride);
+            } else {
+                eq = list_quad(nbl, min(b + 1, nq - 1), i, a.stride);
+            }
 #pragma unroll
             for (int u = 0; u < kB64; ++u) {
                 const double dx = dsub(pi.x, pj[u].x), dy = dsub(pi.y, pj[u].y), dz = dsub(pi.z, pj[u].z);
@@ -504,8 +522,9 @@ __device__ __forceinline__ bool mixed_pair(uint32_t en, const float4& ri, const 
     return !fast && rsq < a.rc2_hi;
 }
 
-template <bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
-__global__ void __launch_bounds__(kThreads, TMD_MINB)
+// AHEAD: the next quad's gathers are in flight while this one's pairs run (force_ahead chooses)
+template <bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false>
+__global__ void __launch_bounds__(kThreads, AHEAD ? 1 : TMD_MINB)
 k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos, float4* __restrict__ frc32,
               double4* __restrict__ vel, const int* __restrict__ nbn, const uint32_t* __restrict__ nbl,
               double* __restrict__ part, LjArgs a, double4* __restrict__ pos_n = nullptr,
@@ -536,13 +555,29 @@ k_lj_mixed_bf(const float4* __restrict__ pos32, const double4* __restrict__ pos,
         // is neither a fast nor a queued pair and the loop needs no count test
         const int nquad = (n + 3) >> 2;
         uint4 eq = n > 0 ? list_quad(nbl, 0, i, a.stride) : make_uint4(0u, 0u, 0u, 0u);
+        uint4 en = AHEAD && nquad > 1 ? list_quad(nbl, 1, i, a.stride) : eq;
+        float4 rn[kB32];
+        auto gather = [&](const uint4& q) {
+            rn[0] = __ldg(pos32 + (q.x >> kCodeBits));
+            rn[1] = __ldg(pos32 + (q.y >> kCodeBits));
+            rn[2] = __ldg(pos32 + (q.z >> kCodeBits));
+            rn[3] = __ldg(pos32 + (q.w >> kCodeBits));
+        };
+        if (AHEAD) gather(eq);
         for (int b = 0; b < nquad; ++b) {
             const uint32_t cur[kB32] = {eq.x, eq.y, eq.z, eq.w};
+            if (!AHEAD) gather(eq);
             float4 rj[kB32];
 #pragma unroll
-            for (int u = 0; u < kB32; ++u) rj[u] = __ldg(pos32 + (cur[u] >> kCodeBits));
-            // the next quad loads while this one's gathers are in flight
-            eq = list_quad(nbl, b + 1, i, a.stride);  // the last read lands in the spare row
+            for (int u = 0; u < kB32; ++u) rj[u] = rn[u];
+            if (AHEAD) {
+                eq = en;
+                gather(eq);
+                en = list_quad(nbl, min(b + 2, nquad - 1), i, a.stride);
+            } else {
+                // the next quad loads while this one's gathers are in flight
+                eq = list_quad(nbl, b + 1, i, a.stride);  // the last read lands in the spare row
+            }
             unsigned slow = 0;
 #pragma unroll
             for (int u = 0; u < kB32; ++u)
@@ -1556,6 +1591,18 @@ int force_lanes(int N, bool mixed) {
     return N <= (mixed ? 29000 : 36000) ? 4 : 1;
 }
 
+// Thread-per-atom kernels with the next quad's gathers in flight.  FP64: 30 % less time per wave of
+// blocks, but five blocks per SM instead of eight, so the numbers of waves decide (step times in us,
+// without / with: 42,592 atoms 25.2 / 22.9, 70,304 28.3 / 26.8, 131,072 44.1 / 50.2, 186,624 73.5 / 59.6,
+// 256,000 84.4 / 84.1, 340,736 114 / 107, 442,368 130 / 133, 702,464 199 / 205).  Mixed: from several
+// waves on, whose blocks start out of step (131,072 34.4 / 34.7, 256,000 70.1 / 71.5, 340,736 88.7 /
+// 86.1, 442,368 111 / 107, 702,464 169 / 163; half-filled box of 524,288 130 / 127).
+bool force_ahead(int N, bool mixed) {
+    if (mixed) return N >= 300000;
+    const int with = nblocks(N, 148 * 5 * kThreads), without = nblocks(N, 148 * 8 * kThreads);
+    return 18 * with < 25 * without;
+}
+
 // blocks of a full-list LJ force launch over N atoms and nchain chain ghosts
 int force_blocks(int N, int lanes, int nchain) {
     if (lanes == 1) return nblocks(N + nchain, kThreads);
@@ -1576,11 +1623,15 @@ void launch_lj_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
 }
 
 // INIT: the kernels write the integrated locals into the other position buffer
-template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
+template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false>
 void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs& pa = PushArgs()) {
+    if constexpr (!HALF && !AHEAD) {
+        if (lanes == 1 && force_ahead(a.N, s.precision == 1))
+            return launch_lj<HALF, FUSE, THERMO, INIT, PUSH, true>(s, a, nb, lanes, pa);
+    }
     double4* vel = s.vel.b[s.vc];
     double4* pn = INIT ? s.pos.b[1 - s.pc] : nullptr;
-    if constexpr (!HALF) {
+    if constexpr (!HALF && !AHEAD) {
         switch (lanes) {
             case 4: return launch_lj_lanes<4, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
             case 8: return launch_lj_lanes<8, FUSE, THERMO, INIT, PUSH>(s, a, nb, pa);
@@ -1593,10 +1644,10 @@ void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs&
             launch(s, nb, kThreads, 0, k_lj_mixed_half<THERMO>, s.pos32.b[s.pc], s.pos.b[s.pc], s.frc32, s.nbn,
                    s.nbl, s.groot, s.red_part, a);
         else
-            launch(s, nb, kThreads, 0, (k_lj_mixed_bf<FUSE, THERMO, INIT, PUSH>), s.pos32.b[s.pc], s.pos.b[s.pc],
+            launch(s, nb, kThreads, 0, (k_lj_mixed_bf<FUSE, THERMO, INIT, PUSH, AHEAD>), s.pos32.b[s.pc], s.pos.b[s.pc],
                    s.frc32, vel, s.nbn, s.nbl, s.red_part, a, pn, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
     } else
-        launch(s, nb, kThreads, 0, (k_lj_fp64<HALF, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac], vel,
+        launch(s, nb, kThreads, 0, (k_lj_fp64<HALF, FUSE, THERMO, INIT, PUSH, AHEAD>), s.pos.b[s.pc], s.frc.b[s.ac], vel,
                s.nbn, s.nbl, s.groot, s.red_part, a, pn, pa);
 }
 

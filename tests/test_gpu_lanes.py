@@ -1,7 +1,7 @@
-"""The LJ force kernels that share an atom between 2 to 16 lanes, on both sides of every size at
-which the number of lanes changes: FP64 bit-identical to the oracle (the pair forces are added in
-list order whatever the lanes), mixed within 1e-5 of the rms force, and the mixed kernels' redo of
-an atom whose FP64-path quads overflow the queue."""
+"""The full-list LJ force kernels on both sides of every size at which the kernel changes (16, 8, 4 lanes
+per atom or one, with and without the next gathers in flight): FP64 bit-identical to the oracle (the
+pair forces are added in list order whatever the lanes), mixed within 1e-5 of the rms force, and the
+mixed kernels with more FP64-path quads than their queue or marks hold."""
 import numpy as np
 import pytest
 
@@ -17,8 +17,10 @@ def thermo(lib):
     return t
 
 
-# 16 | 8 | 4 | 1 lanes: 2,048 | 2,304 and 6,864 | 7,488 and 38,808 | 40,656 atoms
-@pytest.mark.parametrize("cells", [(8, 8, 8), (8, 8, 9), (13, 11, 12), (12, 13, 12), (21, 21, 22), (21, 22, 22)])
+# 16 | 8 | 4 | 1 lanes: 2,048 | 2,304 and 8,112 | 8,216 and 35,912 | 36,960 atoms; one lane with the gathers
+# ahead to 94,720 | without: 94,300 | 97,556; with again: 165,888
+@pytest.mark.parametrize("cells", [(8, 8, 8), (8, 8, 9), (13, 13, 12), (13, 79, 2), (22, 24, 17), (20, 21, 22),
+                                   (28, 29, 29), (29, 29, 29), (36, 36, 32)])
 def test_fp64_bit_identical(product, oracle, cuda_device, cells):
     state = []
     for lib in (product, oracle):
@@ -30,9 +32,10 @@ def test_fp64_bit_identical(product, oracle, cuda_device, cells):
         np.testing.assert_array_equal(a, b)
 
 
-# 16 | 8 | 4 | 2 | 1 lanes: 2,048 | 2,304 and 16,384 | 17,408 and 48,668 | 50,784 and 81,648 | 84,672 atoms
-@pytest.mark.parametrize("cells", [(8, 8, 8), (8, 8, 9), (16, 16, 16), (16, 16, 17), (23, 23, 23), (23, 23, 24),
-                                   (27, 27, 28), (27, 28, 28)])
+# 16 | 8 | 4 | 1 lanes: 1,008 | 1,152 and 8,112 | 9,216 and 28,880 | 30,400 atoms; gathers ahead from 300,000:
+# 299,628 | 303,408
+@pytest.mark.parametrize("cells", [(6, 6, 7), (6, 6, 8), (13, 13, 12), (16, 12, 12), (19, 19, 20), (20, 20, 19),
+                                   (43, 42, 41), (43, 42, 42)])
 def test_mixed_error(product, cuda_device, cells):
     """Forces and sums of the mixed form on the state after 21 steps against the FP64 form's."""
     product.md_set_precision(1)
@@ -56,9 +59,10 @@ def test_mixed_error(product, cuda_device, cells):
     np.testing.assert_allclose(t32[[0, 3]], t64[[0, 3]], rtol=1e-6)
 
 
-# every pair within 1.04 sigma: 8, 4, 2 and 1 lanes with more than 8 queued quads per lane
-@pytest.mark.parametrize("cells,cutoff", [((10, 10, 10), 4.0), ((17, 17, 17), 3.2), ((24, 24, 24), 2.5),
-                                          ((28, 28, 28), 2.5)])
+# every pair within 1.04 sigma, so every quad has FP64-path pairs: 16, 8 and 4 lanes with up to and beyond
+# 64 quads a list, one lane beyond its queue of 8, without and with the gathers ahead
+@pytest.mark.parametrize("cells,cutoff", [((6, 6, 6), 2.5), ((6, 6, 6), 4.0), ((10, 10, 10), 4.0), ((17, 17, 17), 3.2),
+                                          ((17, 17, 17), 4.0), ((24, 24, 24), 2.5), ((43, 42, 42), 2.5)])
 def test_mixed_queue_overflow(product, cuda_device, cells, cutoff):
     product.md_set_precision(1)
     try:
