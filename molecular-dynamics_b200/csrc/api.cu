@@ -427,6 +427,7 @@ size_t list_entries(const State& s) { return (size_t)(s.nb_cap + 4) * s.nb_strid
 void grow_lists(State& s, int rows) {
     dfree(&s.nbl);
     s.nb_cap = list_rows(rows);
+    s.two_short = false;
     dalloc(&s.nbl, list_entries(s));
     s.lists_valid = 0;
 }
@@ -501,6 +502,7 @@ bool require_alive(const char* what) {
 // ---------------------------------------------------------------------------
 void launch_force(State& s, const PendingForce& p, bool fuse_final, double dt) {
     resolve_lists(s);
+    if (!p.half || p.dem || s.precision == 1) one_sided_lists(s);
     s.last_force_half = p.half ? 1 : 0;
     if (p.dem) run_force_dem(s, p);
     else run_force_lj(s, p, fuse_final, dt);
@@ -834,6 +836,7 @@ int md_initialize_grid(double const* masses, Vector3D const* positions, Vector3D
     if (s.halo.on) s.ghost_exact = 1;  // ghosts of other ranks are exact images; own ones likewise
     s.pc = s.vc = s.ac = 0;
     s.lists_valid = 0;
+    s.lists_two = s.two_short = false;
     s.cells_filled = 0;
     s.pend_init = false;
     s.pend_force = PendingForce();
@@ -1352,6 +1355,7 @@ void md_report_iterations(void) {
     long long total = 0;
     if (s.alive) {
         flush_all(s);
+        one_sided_lists(s);
         std::vector<int> n(s.N);
         if (s.N) {
             TMD_CUDA(cudaMemcpyAsync(n.data(), s.nbn, sizeof(int) * s.N, cudaMemcpyDeviceToHost, s.stream));
@@ -1544,6 +1548,7 @@ int md_get_neighbor_lists(int* sizes, int* lists, int capacity) {
     State& s = g_state;
     if (!require_alive("md_get_neighbor_lists")) return -1;
     flush_all(s);
+    one_sided_lists(s);
     const int N = s.N, NA = s.N + s.G;
     std::vector<int> n(N), ref(NA);
     std::vector<uint32_t> l((size_t)s.nb_cap * s.nb_stride);

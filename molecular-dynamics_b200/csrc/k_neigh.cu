@@ -475,6 +475,7 @@ struct NlArgs {
     double cut2;  // cutoff^2 (FP64, the reference's membership test)
     float cut;
     int nbcap, stride, N, ncells, nx, nxy;
+    int two;  // half lists: local pairs from both sides (two_sided)
     double alo[3], spacing;
 };
 
@@ -686,7 +687,8 @@ k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const
                 const int slot = s_slot[min(m, m1 - 1)];
                 const double4 p = ldg_d4(pos + slot);
                 const int kb = __ldg(rbk + slot);
-                if (HM) cref[u] = __ldg(ref + slot);  // root reference index (ref for locals)
+                // root reference index (ref for locals), below every home's where locals always pass
+                if (HM) cref[u] = a.two && slot < a.N ? -1 : __ldg(ref + slot);
                 cp[u] = make_float4((float)(p.x - ox), (float)(p.y - oy), (float)(p.z - oz),
                                     __uint_as_float(((uint32_t)slot << kCodeBits) +
                                                     (uint32_t)(rel_code(kb, rb0) + kCodeBias)));
@@ -931,7 +933,7 @@ k_build_list_sparse(const double4* __restrict__ pos, const int* __restrict__ ref
             slot[u] = m < M ? m + roff : ih;
             p[u] = ldg_d4(pos + slot[u]);
             kb[u] = __ldg(rbk + slot[u]);
-            if (HM) kr[u] = __ldg(ref + slot[u]);
+            if (HM) kr[u] = a.two && slot[u] < a.N ? -1 : __ldg(ref + slot[u]);
         }
 #pragma unroll
         for (int u = 0; u < kSparseBatch; ++u) {
@@ -1412,6 +1414,45 @@ void launch_build_list(State& s, const int* ref, const NlArgs& a, const LinkArgs
     }
 }
 
+// Half lists whose local pairs are held by both atoms (a ghost pair still by one), for the FP64 LJ
+// kernel: it then adds up each atom's own pairs and only a ghost's root gets its reaction by atomics,
+// where three FP64 atomics per pair, 15 M a step at 131,072 atoms, took half of the step; and few atoms
+// can share each atom's list between lanes.  Step times in us, one-sided -> two-sided (boundary pairs
+// kept, rebuild every 20 steps included): 256 atoms 26.8 -> 10.8, 2,048 27.3 -> 11.7, 16,384 28.2 -> 18.9,
+// 48,668 44.3 -> 37.9, 131,072 83.1 -> 57.4, 442,368 240 -> 158, 864,000 447 -> 274.  The list build
+// stays within 2 %.  Not for the other half kernels (DEM's lists are short, the mixed form adds four
+// floats at once), nor where the longer lists outgrow the capacity of the reference's.
+static bool two_sided(const State& s) {
+    return s.precision == 0 && !(s.force_cfg.valid && s.force_cfg.dem) && !s.two_short;
+}
+
+// Drops the entries that the reference's half lists do not hold, in place and in order: a local
+// neighbour stays with the atom of the larger reference index (core/neighborlist.impala:34).
+__global__ void k_one_sided(const int* __restrict__ ref, int* __restrict__ nbn, uint32_t* __restrict__ nbl, int N,
+                            int stride, int nbcap) {
+    const int blk = (int)blockIdx.x + pdl_wait();
+    const int i = blk * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const int n = min(nbn[i], nbcap), iref = ref[i];
+    int out = 0;
+    for (int k = 0; k < n; ++k) {
+        const uint32_t e = nbl[nl_index(k, i, stride)];
+        const int j = (int)(e >> kCodeBits);
+        if (j >= N || ref[j] < iref) nbl[nl_index(out++, i, stride)] = e;
+    }
+    nbn[i] = out;
+    for (; out & 3; ++out) nbl[nl_index(out, i, stride)] = ((uint32_t)i << kCodeBits) | kPadCode;
+}
+
+void one_sided_lists(State& s) {
+    if (!s.lists_two) return;
+    resolve_lists(s);
+    if (!s.lists_two) return;  // they outgrew the capacity and were built again
+    s.lists_two = false;
+    launch(s, nblocks(s.N, 256), 256, 0, k_one_sided, s.ref.b[s.ac], s.nbn, s.nbl, s.N, s.nb_stride, s.nb_cap);
+    launched(K_NLIST);
+}
+
 // A list build's status, read back: the locals outside the grid get empty lists, the two-phase
 // chain and image-map state of the links; 0 when the lists stand, 1 when the capacity was short
 // (grown: the build is to be redone).
@@ -1436,6 +1477,10 @@ static int finish_build(State& s, bool half) {
         s.lists_half = half;
         return 0;
     }
+    if (s.lists_two) {  // one-sided lists may still fit
+        s.two_short = true;
+        return 1;
+    }
     // core/neighborlist.impala:74-76: grow to twice the overflow and redo
     std::printf("0> reallocate_neighborlist_capacity(): %d\n", mx * 2);
     grow_lists(s, mx * 2);
@@ -1447,6 +1492,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     s.lists_cutoff = cutoff;
     s.status_pending = false;
     if (s.N == 0) {
+        s.lists_two = false;
         s.lists_valid = 1;
         s.lists_half = half;
         return 0;
@@ -1466,6 +1512,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     a.spacing = g.spacing;
     for (int attempt = 0; attempt < 8; ++attempt) {
         a.nbcap = s.nb_cap;
+        a.two = s.lists_two = half && two_sided(s);
         if (attempt > 0 || !s.build_zeroed)  // else zeroed by the binning's reorder kernel
             TMD_CUDA(cudaMemsetAsync(&s.status_dev->max_nb, 0, sizeof(int), s.stream));
         s.build_zeroed = false;

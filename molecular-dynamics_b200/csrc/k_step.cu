@@ -181,7 +181,9 @@ __device__ __forceinline__ void push_chain(int q, const double4* __restrict__ po
 // PUSH (with INIT): the kernel also writes the ghosts (PushArgs)
 // AHEAD: the next quad's gathers are in flight while this one's pairs run; its registers leave five
 // blocks per SM instead of eight (force_ahead chooses)
-template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false>
+// TWO (with HALF): both atoms of a local pair hold it, so reactions go to the ghosts' roots only
+template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false,
+          bool TWO = false>
 __global__ void __launch_bounds__(kThreads)
 k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
           const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, const int* __restrict__ groot,
@@ -241,16 +243,17 @@ k_lj_fp64(const double4* __restrict__ pos, double4* __restrict__ frc, double4* _
                     fx = dadd(fx, px);
                     fy = dadd(fy, py);
                     fz = dadd(fz, pz);
-                    if (HALF) {
+                    if (HALF && (!TWO || j[u] >= a.N)) {
                         const int t = reaction_slot(j[u], a.N, groot);
                         atomicAdd(&frc[t].x, -px);
                         atomicAdd(&frc[t].y, -py);
                         atomicAdd(&frc[t].z, -pz);
                     }
                     if (THERMO) {
-                        e += 4.0 * a.eps * sr6 * (sr6 - 1.0);
-                        w += f * rsq;
-                        cnt += 1.0;
+                        const double seen = TWO && j[u] < a.N ? 0.5 : 1.0;
+                        e += seen * (4.0 * a.eps * sr6 * (sr6 - 1.0));
+                        w += seen * (f * rsq);
+                        cnt += seen;
                     }
                 }
             }
@@ -867,11 +870,13 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
 // and three lanes of the atom add one component each, in order, while the next round's quads load.
 // An entry outside the cutoff or past the list's end adds +0.0, which changes no bit of a sum that
 // starts at +0.0 (such a sum is never -0.0).
-template <int L, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false>
+// TWO: half lists whose local pairs both atoms hold, as in k_lj_fp64
+template <int L, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool TWO = false>
 __global__ void __launch_bounds__(kThreads)
 k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, double4* __restrict__ vel,
                 const int* __restrict__ nbn, const uint32_t* __restrict__ nbl, double* __restrict__ part, LjArgs a,
-                int atom_blocks, double4* __restrict__ pos_n = nullptr, PushArgs pa = PushArgs()) {
+                int atom_blocks, double4* __restrict__ pos_n = nullptr, PushArgs pa = PushArgs(),
+                const int* __restrict__ groot = nullptr) {
     const int blk = (int)blockIdx.x + pdl_wait();
     static_assert(L >= 4 && L <= 32, "three lanes of an atom add its force's components");
     // pairs outside the cutoff evaluated too, without a branch: shorter chains (2,048 atoms, 8 lanes:
@@ -911,6 +916,8 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
         if (kAhead) gather(eq);
         for (int r = 0; r < rounds; ++r) {
             const int b = r * L + sub;
+            const int j[kB64] = {(int)(eq.x >> kCodeBits), (int)(eq.y >> kCodeBits), (int)(eq.z >> kCodeBits),
+                                 (int)(eq.w >> kCodeBits)};
             if (!kAhead) {
                 gather(eq);
                 eq = en;
@@ -931,10 +938,17 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
                 p[0][u] = in ? dmul(dx, f) : 0.0;
                 p[1][u] = in ? dmul(dy, f) : 0.0;
                 p[2][u] = in ? dmul(dz, f) : 0.0;
+                if (TWO && in && j[u] >= a.N) {
+                    double4* to = frc + groot[j[u] - a.N];
+                    atomicAdd(&to->x, -p[0][u]);
+                    atomicAdd(&to->y, -p[1][u]);
+                    atomicAdd(&to->z, -p[2][u]);
+                }
                 if (THERMO && in) {
-                    e += 4.0 * a.eps * sr6 * (sr6 - 1.0);
-                    w += f * rsq;
-                    cnt += 1.0;
+                    const double seen = TWO && j[u] < a.N ? 0.5 : 1.0;
+                    e += seen * (4.0 * a.eps * sr6 * (sr6 - 1.0));
+                    w += seen * (f * rsq);
+                    cnt += seen;
                 }
             }
             // entry 4 sub + 2 h + e of the round at h 2 L + 2 sub + e
@@ -964,7 +978,11 @@ k_lj_fp64_lanes(const double4* __restrict__ pos, double4* __restrict__ frc, doub
         const int base = lane & ~(L - 1);
         const double fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
                      fz = __shfl_sync(0xffffffffu, acc, base + 2);
-        if (act && sub == 0) st_d4(frc + i, make_double4(fx, fy, fz, 0.0));
+        if (TWO) {
+            if (act && sub < 3) atomicAdd(&frc[i].x + sub, acc);
+        } else if (act && sub == 0) {
+            st_d4(frc + i, make_double4(fx, fy, fz, 0.0));
+        }
         if (FUSE) {  // core/compute.impala:108-116
             double4 v = act ? ld_d4(vel + i) : make_double4(0.0, 0.0, 0.0, 0.0);
             v.x = dadd(v.x, dmul(fx, a.h));
@@ -1619,12 +1637,34 @@ void launch_lj_lanes(State& s, const LjArgs& a, int nb, const PushArgs& pa) {
                s.frc32, vel, s.nbn, s.nbl, s.red_part, a, ab, pn, INIT ? s.pos32.b[1 - s.pc] : nullptr, s.rbk, pa);
     else
         launch(s, nb, kThreads, 0, (k_lj_fp64_lanes<L, FUSE, THERMO, INIT, PUSH>), s.pos.b[s.pc], s.frc.b[s.ac], vel,
-               s.nbn, s.nbl, s.red_part, a, ab, pn, pa);
+               s.nbn, s.nbl, s.red_part, a, ab, pn, pa, nullptr);
 }
 
 // INIT: the kernels write the integrated locals into the other position buffer
 template <bool HALF, bool FUSE, bool THERMO, bool INIT = false, bool PUSH = false, bool AHEAD = false>
 void launch_lj(State& s, const LjArgs& a, int nb, int lanes = 1, const PushArgs& pa = PushArgs()) {
+    if constexpr (HALF) {
+        if (s.lists_two) {  // FP64 (launch_force)
+            const int ab = nblocks((long long)a.N * lanes, kThreads);
+            auto by_lanes = [&](auto kernel) {
+                launch(s, nb, kThreads, 0, kernel, s.pos.b[s.pc], s.frc.b[s.ac], nullptr, s.nbn, s.nbl, s.red_part, a, ab,
+                       nullptr, pa, s.groot);
+            };
+            auto by_atom = [&](auto kernel) {
+                launch(s, nb, kThreads, 0, kernel, s.pos.b[s.pc], s.frc.b[s.ac], nullptr, s.nbn, s.nbl, s.groot,
+                       s.red_part, a, nullptr, pa);
+            };
+            switch (lanes) {
+                case 4: return by_lanes(k_lj_fp64_lanes<4, false, THERMO, false, false, true>);
+                case 8: return by_lanes(k_lj_fp64_lanes<8, false, THERMO, false, false, true>);
+                case 16: return by_lanes(k_lj_fp64_lanes<16, false, THERMO, false, false, true>);
+                default: break;
+            }
+            if (force_ahead(a.N, false)) by_atom(k_lj_fp64<true, false, THERMO, false, false, true, true>);
+            else by_atom(k_lj_fp64<true, false, THERMO, false, false, false, true>);
+            return;
+        }
+    }
     if constexpr (!HALF && !AHEAD) {
         if (lanes == 1 && force_ahead(a.N, s.precision == 1))
             return launch_lj<HALF, FUSE, THERMO, INIT, PUSH, true>(s, a, nb, lanes, pa);
@@ -1710,7 +1750,7 @@ void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt) {
     a.hy = (float)(-s.geo.rb_h / 4.0);
     a.hz = (float)(-s.geo.rb_h / 16.0);
     const bool half = p.half;
-    const int lanes = half ? 1 : force_lanes(N, s.precision == 1);
+    const int lanes = half && !s.lists_two ? 1 : force_lanes(N, s.precision == 1);
     const int nb = force_blocks(N, lanes, 0);
     const bool thermo = s.thermo != 0;
     if (thermo) {
@@ -1727,8 +1767,8 @@ void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt) {
     }
     prof_begin(K_FORCE_LJ);
     if (half) {
-        if (thermo) launch_lj<true, false, true>(s, a, nb);
-        else launch_lj<true, false, false>(s, a, nb);
+        if (thermo) launch_lj<true, false, true>(s, a, nb, lanes);
+        else launch_lj<true, false, false>(s, a, nb, lanes);
     } else if (fuse_final) {
         if (thermo) launch_lj<false, true, true>(s, a, nb, lanes);
         else launch_lj<false, true, false>(s, a, nb, lanes);

@@ -169,6 +169,8 @@ struct State {
     int nblk_border = 0;
     int lists_valid = 0;
     bool lists_half = false;
+    bool lists_two = false;   // half lists that hold their local pairs from both sides (two_sided, k_neigh.cu)
+    bool two_short = false;   // such lists outgrew the capacity: one-sided builds until it changes
     int max_list = 0;      // longest list of the last build whose status was read
     int cells_filled = 0;  // cells that hold locals, at the last binning whose status was read (0: none)
 
@@ -322,6 +324,7 @@ void run_borders(State& s, bool wrap = false);   // ghost generation, reference 
 void run_distribute(State& s);                    // binning + reorder
 // defer: the status readback is left in flight (resolve_lists completes it)
 int run_build_lists(State& s, bool half, double cutoff, bool defer = false);  // returns 0 or error
+void one_sided_lists(State& s);  // half lists as the reference holds them (no-op when they are)
 // completes a deferred list build: 0 when the lists stand, 1 when they were rebuilt (a force
 // kernel launched on them speculatively returned without writing), -1 on an error
 int resolve_lists(State& s);
