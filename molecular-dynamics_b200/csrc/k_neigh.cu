@@ -3,9 +3,10 @@
 //   * ghost generation (borders)     (comm/comm.impala:105-127, 528-642, 723-734; comm/lb.impala:88-100)
 //   * cell binning as a counting sort that reorders the device arrays by cell
 //                                    (core/grid.impala:280-321, 406-426)
-//   * neighbour-list build, one warp per cell with a home atom per lane, the
-//     stencil's candidates filtered by the homes' bounding box and staged in
-//     shared memory               (core/neighborlist.impala:1-78)
+//   * neighbour-list build (core/neighborlist.impala:1-78): a block per cell,
+//     the stencil's candidates filtered by the homes' bounding box and staged
+//     in shared memory, a warp testing 32 of them against a home at once; or
+//     eight lanes per home where cells hold few atoms
 //
 // Ghost order.  The reference runs six passes (x+, x-, y+, y-, z+, z-); a
 // pass scans locals then all earlier ghosts in order and appends the ones
@@ -450,11 +451,14 @@ __device__ __forceinline__ bool exact_within(const double4* __restrict__ pos, in
 // so membership is exactly the reference's; the FP32 margin follows from the magnitude of the staged
 // coordinates (margin32), which makes that test rare.
 //
-// Bound by instruction issue (75 %): 67 M warp instructions at 131,072 atoms, 41 M of them the 1.4 M
-// steps of 32 pair tests, the rest the staging.  One warp per cell with a home per lane walking the
+// Bound by instruction issue (77 %): 67 M warp instructions at 131,072 atoms, 46 M of them the pair
+// tests, 16 M the staging, 5 M the blocks' start; without the tests the kernel takes 36 of 85 us, without
+// the staging too 18 us (the chain of loads and barriers that starts a block).  One warp per cell with a home per lane walking the
 // candidates one by one, as this kernel did before, took 83 M (19 of 32 lanes held a home) and made
 // small systems wait for one serial walk.  Measured before -> now (us): 256 atoms 43 -> 15, 2,048
-// 48 -> 18, 16,384 51 -> 23, 131,072 124 -> 91, 442,368 336 -> 268; half lists at 131,072 167 -> 102.
+// 48 -> 18, 16,384 51 -> 23, 131,072 124 -> 91, 442,368 336 -> 268; half lists at 131,072 167 -> 102
+// (105 where they hold their local pairs from both sides).  More blocks per SM: 98-104 us at 131,072 with 9, 10
+// or 12 (56, 48, 40 registers: spills).
 // A step of 1, 3 or 4 chunks instead of 2: 97, 92, 96 us at 131,072; the FP64 test or the emptying of
 // a full buffer inside the step loop, where the compiler predicates it: 130 us.
 //

@@ -9,9 +9,10 @@
 //   * stand-alone ghost refresh and final integration
 //   * deterministic FP64 reductions of energy, virial and kinetic energy
 //
-// Thread per local atom; the atom-fastest list makes the index loads of a
-// warp one coalesced 128-byte line per neighbour slot, and neighbour
-// positions come through the read-only path.
+// Thread per local atom in a large system, 4 to 16 lanes per atom in a small
+// one (force_lanes, dem_lanes); the list's quads of four entries, atom-fastest,
+// make a warp's index loads one coalesced 512-byte line per quad, and neighbour
+// positions come through the read-only path, an FP64 position in one 256-bit load.
 
 #include "launch.cuh"
 #include "lj_args.cuh"
