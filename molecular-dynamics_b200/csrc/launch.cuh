@@ -40,7 +40,8 @@ inline void launch(const State& s, unsigned grid, unsigned block, size_t shared,
     c.dynamicSmemBytes = shared;
     c.stream = s.stream;
     c.attrs = &at;
-    c.numAttrs = s.stream ? 1 : 0;  // the legacy default stream keeps plain launches
+    // the default streams, by NULL or by their handles, keep plain launches
+    c.numAttrs = s.stream && s.stream != cudaStreamLegacy && s.stream != cudaStreamPerThread ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 

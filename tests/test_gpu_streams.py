@@ -44,3 +44,12 @@ def test_callers_streams(product, oracle, cuda_device, stream):
     script = SCRIPT.format(pkg=PKG, tests=os.path.join(ROOT, "tests"), stream=stream)
     r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("handle", [1, 2])
+def test_default_stream_handles(product, oracle, cuda_device, handle):
+    """The legacy and per-thread default streams by their handles."""
+    script = SCRIPT.format(pkg=PKG, tests=os.path.join(ROOT, "tests"), stream="None").replace(
+        "stream.cuda_stream if stream else 0", str(handle)).replace("a.add_(1.0)", "a.add_(1.0); torch.cuda.synchronize()")
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
