@@ -341,18 +341,12 @@ std::vector<SlabItem> slab_items(State& s) {
     return v;
 }
 
-// the events and the copy stream of a grid
+// the events of a grid
 void free_sync_objects(State& s) {
-    for (cudaEvent_t* e : {&s.ev_counted, &s.ev_scanned, &s.ev_status}) {
-        if (*e) cudaEventDestroy(*e);
-        *e = nullptr;
-    }
     for (cudaEvent_t& e : s.thermo_ev) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
     }
-    if (s.copy_stream) cudaStreamDestroy(s.copy_stream);
-    s.copy_stream = nullptr;
     s.sync_device = -1;
 }
 
@@ -368,10 +362,9 @@ void free_all(State& s) {
     dfree(&s.bmask);
     dfree(&s.nbl);
     dfree(&s.red_part);
-    // the events and the copy stream stay for the next grid (made anew when the device changes)
-    if (s.ev_status) cudaEventSynchronize(s.ev_status);
+    // the events stay for the next grid (made anew when the device changes)
+    if (s.status_pending) await_word(s, &s.status_host->ready);
     s.status_pending = false;
-    if (s.copy_stream) cudaStreamSynchronize(s.copy_stream);
     for (int k = 0; k < kThermoSlots; ++k) s.thermo_slot_ticket[k] = -1;
     dfree(&s.thermo_dev);
     dfree(&s.status_dev);
@@ -469,17 +462,13 @@ bool allocate_state(State& s, int N, int nb_cap) {
     dalloc(&s.nbl, list_entries(s));
     if (s.sync_device != s.device) {
         free_sync_objects(s);
-        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_counted, cudaEventDisableTiming));
-        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_scanned, cudaEventDisableTiming));
-        TMD_CUDA(cudaEventCreateWithFlags(&s.ev_status, cudaEventDisableTiming));
-        TMD_CUDA(cudaStreamCreateWithFlags(&s.copy_stream, cudaStreamNonBlocking));
         for (int k = 0; k < kThermoSlots; ++k)
             TMD_CUDA(cudaEventCreateWithFlags(&s.thermo_ev[k], cudaEventDisableTiming));
         s.sync_device = s.device;
     }
     dalloc(&s.thermo_dev, 8);
     dalloc(&s.status_dev, 1);
-    if (!s.status_host) TMD_CUDA(cudaMallocHost((void**)&s.status_host, sizeof(DevStatus)));
+    if (!s.status_host) TMD_CUDA(cudaMallocHost((void**)&s.status_host, sizeof(HostStatus)));
     if (!s.thermo_host) TMD_CUDA(cudaMallocHost((void**)&s.thermo_host, kThermoSlots * 4 * sizeof(double)));
     for (int k = 0; k < kThermoSlots; ++k) s.thermo_slot_ticket[k] = -1;
     s.thermo_tickets = 0;

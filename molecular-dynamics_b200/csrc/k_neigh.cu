@@ -23,6 +23,8 @@
 // which makes list order -- and hence FP64 force summation order -- equal to
 // the reference's.
 
+#include <atomic>
+#include <chrono>
 #include <cstdio>
 
 #include "comm.h"
@@ -194,8 +196,13 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
                               const unsigned* __restrict__ bmask, const int* __restrict__ boff,
                               int* __restrict__ gsrc, int* __restrict__ groot, int* __restrict__ gcode,
                               int* __restrict__ bsrc_ref, int* __restrict__ broot_ref, int* __restrict__ bcode,
-                              int N, int nblk, int capA, GeoArgs a, int sync_vel, RemoteOut ro) {
+                              int N, int nblk, int capA, GeoArgs a, int sync_vel, RemoteOut ro,
+                              int* count_host) {
     const int blk = (int)blockIdx.x + pdl_wait();
+    if (count_host && blk == 0 && threadIdx.x == 0) {  // the ghost count, to the host that polls for it
+        *reinterpret_cast<volatile int*>(count_host) = boff[26 * nblk];
+        __threadfence_system();
+    }
     __shared__ int wpre[kBorderThreads / 32][26];
     __shared__ unsigned char s_rank[26][kBorderThreads];  // a thread's rank among its warp's ghosts of each type
     const int r = blk * blockDim.x + threadIdx.x;
@@ -1231,6 +1238,23 @@ void run_enforce_pbc(State& s) {
 
 bool grow_atoms(State& s, int need);  // api.cu
 
+// A word of HostStatus that a kernel in flight stores, polled for: the host goes on a few microseconds
+// earlier than after a copy and an event, and the kernels keep following one another without either
+// between them.  When it does not come (a failed launch, a long queue ahead) the stream's work is
+// waited for.  A rebuild of eight kernels with two such waits, by copies and events -> by words stored (us
+// on top of an ordinary step): 256 atoms 54 -> 43, 2,048 55 -> 42, 16,384 65 -> 54, 131,072 143 -> 133,
+// half-filled box of 524,288 433 -> 422, granular gas of 260,800 162 -> 149; at a rebuild every 20 steps
+// 7.24 -> 6.65 us a step at 256 atoms, 14.0 -> 13.6 at 16,384, 44.4 -> 43.75 at 131,072.
+bool await_word(State& s, int* word) {
+    volatile int* const w = word;
+    const auto start = std::chrono::steady_clock::now();
+    for (unsigned polls = 1; *w < 0; ++polls)
+        if ((polls & 0xfffu) == 0 && std::chrono::steady_clock::now() - start > std::chrono::seconds(1)) break;
+    if (*w < 0) TMD_CUDA(cudaStreamSynchronize(s.stream));
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return *w >= 0;
+}
+
 void run_borders(State& s, bool wrap) {
     GeoArgs a = geo_args(s.geo);
     const int N = s.N;
@@ -1265,7 +1289,7 @@ void run_borders(State& s, bool wrap) {
             RemoteOut ro{s.halo.tab, s.halo.send_ref, s.halo.send_type, comm().topo.selfmask};
             launch(s, nblk, kBorderThreads, 0, k_border_emit<true>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
                    s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot, s.gcode, s.bsrc_ref,
-                   s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, ro);
+                   s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, ro, nullptr);
             launched(K_BORDER);
         }
         if (ok) ok = halo_finish_borders(s);
@@ -1287,21 +1311,23 @@ void run_borders(State& s, bool wrap) {
     // slots below the capacity, so when the count shows the capacity was short the host
     // grows the arrays (which waits for that emit) and emits again.  The host thus enqueues
     // the next kernels before emit finishes instead of leaving the GPU idle for a round trip.
-    // The readback runs on a second stream, so the emit kernel does not queue behind the copy
-    // (a rebuild's ghost phase 40 -> 33 us at 131k atoms).
-    TMD_CUDA(cudaEventRecord(s.ev_scanned, s.stream));
-    TMD_CUDA(cudaStreamWaitEvent(s.copy_stream, s.ev_scanned, 0));
-    TMD_CUDA(cudaMemcpyAsync(&s.status_host->nghost, boff + n, sizeof(int), cudaMemcpyDeviceToHost, s.copy_stream));
-    TMD_CUDA(cudaEventRecord(s.ev_counted, s.copy_stream));
-    auto emit = [&]() {
+    // Emit's first thread stores the count straight to page-locked memory (await_word).
+    auto emit = [&](int* count) {
         launch(s, nblk, kBorderThreads, 0, k_border_emit<false>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
                s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot, s.gcode, s.bsrc_ref,
-               s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, RemoteOut{nullptr, nullptr, nullptr, 0u});
+               s.broot_ref, s.bcode, N, nblk, s.capA, a, s.dem_fixed, RemoteOut{nullptr, nullptr, nullptr, 0u}, count);
         launched(K_BORDER);
     };
-    emit();
-    TMD_CUDA(cudaEventSynchronize(s.ev_counted));
-    const int G = s.status_host->nghost;
+    int* const count = &s.status_host->nghost;
+    *static_cast<volatile int*>(count) = -1;
+    emit(count);
+    if (!await_word(s, count)) {  // a latched error
+        s.G = 0;
+        s.lists_valid = 0;
+        prof_end(K_BORDER);
+        return;
+    }
+    const int G = *static_cast<volatile int*>(count);
     if (N + G > s.capA) {
         if (!grow_atoms(s, N + G)) {  // no room: no ghosts rather than writes past the arrays
             s.G = 0;
@@ -1309,7 +1335,7 @@ void run_borders(State& s, bool wrap) {
             prof_end(K_BORDER);
             return;
         }
-        emit();
+        emit(nullptr);
     }
     prof_end(K_BORDER);
     s.G = G;
@@ -1457,12 +1483,23 @@ void one_sided_lists(State& s) {
     launched(K_NLIST);
 }
 
+// the list build's status to the host
+__global__ void k_status_out(const DevStatus* st, HostStatus* out) {
+    const int blk = (int)blockIdx.x + pdl_wait();
+    constexpr int kWords = sizeof(DevStatus) / sizeof(int);
+    const int t = threadIdx.x + blk;
+    if (t < kWords) reinterpret_cast<volatile int*>(&out->build)[t] = reinterpret_cast<const volatile int*>(st)[t];
+    __threadfence_system();
+    __syncwarp();
+    if (t == 0) *reinterpret_cast<volatile int*>(&out->ready) = 1;
+}
+
 // A list build's status, read back: the locals outside the grid get empty lists, the two-phase
 // chain and image-map state of the links; 0 when the lists stand, 1 when the capacity was short
 // (grown: the build is to be redone).
 static int finish_build(State& s, bool half) {
     const Geometry& g = s.geo;
-    if (s.status_host->out_local > 0) {
+    if (s.status_host->build.out_local > 0) {
         int first_out = 0;
         // locals outside the grid sit at [cstart[ncells], N): empty lists
         TMD_CUDA(cudaMemcpyAsync(&first_out, s.cstart + g.ncells, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
@@ -1471,10 +1508,10 @@ static int finish_build(State& s, bool half) {
         launched(K_NLIST);
         set_error(5, "locals outside the cell grid at binning (they have no neighbours)");
     }
-    s.nchain = s.status_host->nchain;
-    s.cells_filled = s.status_host->filled;
-    s.img_ok = (s.status_host->img_over1 == 0 ? 1 : 0) | (s.status_host->img_over2 == 0 ? 2 : 0);
-    const int mx = s.status_host->max_nb;
+    s.nchain = s.status_host->build.nchain;
+    s.cells_filled = s.status_host->build.filled;
+    s.img_ok = (s.status_host->build.img_over1 == 0 ? 1 : 0) | (s.status_host->build.img_over2 == 0 ? 2 : 0);
+    const int mx = s.status_host->build.max_nb;
     s.max_list = mx;
     if (mx <= s.nb_cap) {
         s.lists_valid = 1;
@@ -1530,11 +1567,12 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
         else launch_build_list<0>(s, s.ref.b[s.ac], a, la, links);
         launched(K_NLIST);
         prof_end(K_NLIST);
-        TMD_CUDA(cudaMemcpyAsync(s.status_host, s.status_dev, sizeof(DevStatus), cudaMemcpyDeviceToHost, s.stream));
+        *static_cast<volatile int*>(&s.status_host->ready) = -1;
+        launch(s, 1, 32, 0, k_status_out, s.status_dev, s.status_host);
+        launched(K_MISC);
         if (defer && attempt == 0) {
             // the host goes on; the next force kernel is launched on these lists at once and
             // resolve_lists reads the status while it runs
-            TMD_CUDA(cudaEventRecord(s.ev_status, s.stream));
             s.status_pending = true;
             s.status_half = half;
             s.lists_valid = 0;
@@ -1550,8 +1588,8 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
 int resolve_lists(State& s) {
     if (!s.status_pending) return 0;
     s.status_pending = false;
-    TMD_CUDA(cudaEventSynchronize(s.ev_status));
-    const bool outside = s.status_host->out_local > 0;
+    if (!await_word(s, &s.status_host->ready)) return -1;  // a latched error
+    const bool outside = s.status_host->build.out_local > 0;
     if (finish_build(s, s.status_half) == 0) return outside ? 1 : 0;
     // the capacity was short: the build again, on the grown lists
     return run_build_lists(s, s.status_half, s.lists_cutoff) == 0 ? 1 : -1;

@@ -90,9 +90,8 @@ struct Geometry {
     double rb_h;
 };
 
-// Device-side status words written by kernels and read back with one copy.
+// Device-side status words written by kernels; a one-warp kernel hands them to the host (HostStatus).
 struct DevStatus {
-    int nghost;         // ghosts produced by the last border pass
     // zeroed together before a binning (one memset): out_local .. filled
     int out_local;      // locals outside the cell grid at the last binning
     int out_ghost;      // ghosts outside the cell grid
@@ -101,6 +100,13 @@ struct DevStatus {
     int img_over2;      // locals with more than kImg2 images in all
     int filled;         // cells that hold locals
     int max_nb;         // longest neighbour list of the last build (zeroed before each build)
+};
+
+// Page-locked words that kernels store straight to and the host polls (await_word): -1 before.
+struct HostStatus {
+    DevStatus build;  // of the last list build, valid once `ready` is 1
+    int ready;
+    int nghost;       // ghosts of the border pass in flight
 };
 
 // periodic images a local can push (two-phase: its own first-pass images, one per face
@@ -229,18 +235,14 @@ struct State {
     // comes back while the next force kernel already runs: resolve_lists reads it.
     bool status_pending = false;
     bool status_half = false;  // the pending build's list mode (a redo after a capacity growth)
-    cudaEvent_t ev_status = nullptr;
     // scan scratch, reductions, status
     int* scan_part = nullptr;  int scan_part_cap = 0;
     double* red_part = nullptr; int red_part_cap = 0;
     int red_nb = 0, red_q0 = 0, red_q1 = 0;  // quantities [red_q0, red_q1) of red_nb blocks wait there for flush_thermo
     double* thermo_dev = nullptr;   // [8]
     DevStatus* status_dev = nullptr;
-    DevStatus* status_host = nullptr;  // pinned
-    cudaEvent_t ev_counted = nullptr;  // the ghost count's readback (run_borders)
-    cudaEvent_t ev_scanned = nullptr;  // the ghost offsets scanned (the readback waits on it)
-    cudaStream_t copy_stream = nullptr;  // the ghost count's readback, beside the emit kernel
-    int sync_device = -1;              // device whose events and copy stream the grid holds (kept between grids)
+    HostStatus* status_host = nullptr;  // pinned
+    int sync_device = -1;              // device whose events the grid holds (kept between grids)
     int scan_attr_device = -1;         // device whose k_scan_single shared-memory attribute is set
     unsigned long long* lb_tiles = nullptr;  // look-back scan: one word per tile (k_neigh.cu)
     int lb_tile_cap = 0;
@@ -328,6 +330,7 @@ void one_sided_lists(State& s);  // half lists as the reference holds them (no-o
 // completes a deferred list build: 0 when the lists stand, 1 when they were rebuilt (a force
 // kernel launched on them speculatively returned without writing), -1 on an error
 int resolve_lists(State& s);
+bool await_word(State& s, int* word);  // false: still -1 after the stream's work
 void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt);
 void run_force_dem(State& s, const PendingForce& p);
 // kick_dt >= 0: the previous step's final kick of kick_dt is applied first (held back by

@@ -53,3 +53,12 @@ def test_default_stream_handles(product, oracle, cuda_device, handle):
         "stream.cuda_stream if stream else 0", str(handle)).replace("a.add_(1.0)", "a.add_(1.0); torch.cuda.synchronize()")
     r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
+
+
+def test_rebuild_behind_a_long_queue(product, oracle, cuda_device):
+    """The ghost count and the list status that the host polls for come late: over a second of the
+    caller's work on the same stream is ahead of every rebuild's kernels in the first steps."""
+    script = SCRIPT.format(pkg=PKG, tests=os.path.join(ROOT, "tests"), stream="torch.cuda.Stream()").replace(
+        "a.add_(1.0)", "a.add_(1.0); k < 3 and torch.cuda._sleep(int(1.6e9))")
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stdout + r.stderr
