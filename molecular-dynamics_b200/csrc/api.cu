@@ -363,7 +363,7 @@ void free_all(State& s) {
     dfree(&s.nbl);
     dfree(&s.red_part);
     // the events stay for the next grid (made anew when the device changes)
-    if (s.status_pending) await_word(s, &s.status_host->ready);
+    if (s.status_pending) await_words(s, &s.status_host->build, kStatusWords);
     s.status_pending = false;
     for (int k = 0; k < kThermoSlots; ++k) s.thermo_slot_ticket[k] = -1;
     dfree(&s.thermo_dev);

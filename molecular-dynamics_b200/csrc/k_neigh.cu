@@ -199,10 +199,8 @@ __global__ void __launch_bounds__(kBorderThreads) k_border_emit(double4* __restr
                               int N, int nblk, int capA, GeoArgs a, int sync_vel, RemoteOut ro,
                               int* count_host) {
     const int blk = (int)blockIdx.x + pdl_wait();
-    if (count_host && blk == 0 && threadIdx.x == 0) {  // the ghost count, to the host that polls for it
+    if (count_host && blk == 0 && threadIdx.x == 0)  // the ghost count, to the host that polls for it
         *reinterpret_cast<volatile int*>(count_host) = boff[26 * nblk];
-        __threadfence_system();
-    }
     __shared__ int wpre[kBorderThreads / 32][26];
     __shared__ unsigned char s_rank[26][kBorderThreads];  // a thread's rank among its warp's ghosts of each type
     const int r = blk * blockDim.x + threadIdx.x;
@@ -1238,21 +1236,25 @@ void run_enforce_pbc(State& s) {
 
 bool grow_atoms(State& s, int need);  // api.cu
 
-// A word of HostStatus that a kernel in flight stores, polled for: the host goes on a few microseconds
+// Words of HostStatus that a kernel in flight stores, polled for: the host goes on a few microseconds
 // earlier than after a copy and an event, and the kernels keep following one another without either
-// between them.  When it does not come (a failed launch, a long queue ahead) the stream's work is
+// between them.  When they do not come (a failed launch, a long queue ahead) the stream's work is
 // waited for.  A rebuild of eight kernels with two such waits, by copies and events -> by words stored (us
 // on top of an ordinary step): 256 atoms 54 -> 43, 2,048 55 -> 42, 16,384 65 -> 54, 131,072 143 -> 133,
 // half-filled box of 524,288 433 -> 422, granular gas of 260,800 162 -> 149; at a rebuild every 20 steps
 // 7.24 -> 6.65 us a step at 256 atoms, 14.0 -> 13.6 at 16,384, 44.4 -> 43.75 at 131,072.
-bool await_word(State& s, int* word) {
-    volatile int* const w = word;
+bool await_words(State& s, void* words, int n) {
+    const volatile int* const w = static_cast<const volatile int*>(words);
     const auto start = std::chrono::steady_clock::now();
-    for (unsigned polls = 1; *w < 0; ++polls)
+    int k = 0;
+    for (unsigned polls = 1; k < n; ++polls) {
+        while (k < n && w[k] >= 0) ++k;
         if ((polls & 0xfffu) == 0 && std::chrono::steady_clock::now() - start > std::chrono::seconds(1)) break;
-    if (*w < 0) TMD_CUDA(cudaStreamSynchronize(s.stream));
+    }
+    if (k < n) TMD_CUDA(cudaStreamSynchronize(s.stream));
     std::atomic_thread_fence(std::memory_order_acquire);
-    return *w >= 0;
+    while (k < n && w[k] >= 0) ++k;
+    return k == n;
 }
 
 void run_borders(State& s, bool wrap) {
@@ -1311,7 +1313,7 @@ void run_borders(State& s, bool wrap) {
     // slots below the capacity, so when the count shows the capacity was short the host
     // grows the arrays (which waits for that emit) and emits again.  The host thus enqueues
     // the next kernels before emit finishes instead of leaving the GPU idle for a round trip.
-    // Emit's first thread stores the count straight to page-locked memory (await_word).
+    // Emit's first thread stores the count straight to page-locked memory (await_words).
     auto emit = [&](int* count) {
         launch(s, nblk, kBorderThreads, 0, k_border_emit<false>, s.pos.b[s.pc], s.vel.b[s.vc], s.frc.b[s.ac],
                s.mass.b[s.ac], s.ref.b[s.ac], s.slot_of_ref, s.bmask, boff, s.gsrc, s.groot, s.gcode, s.bsrc_ref,
@@ -1321,7 +1323,7 @@ void run_borders(State& s, bool wrap) {
     int* const count = &s.status_host->nghost;
     *static_cast<volatile int*>(count) = -1;
     emit(count);
-    if (!await_word(s, count)) {  // a latched error
+    if (!await_words(s, count, 1)) {  // a latched error
         s.G = 0;
         s.lists_valid = 0;
         prof_end(K_BORDER);
@@ -1486,12 +1488,8 @@ void one_sided_lists(State& s) {
 // the list build's status to the host
 __global__ void k_status_out(const DevStatus* st, HostStatus* out) {
     const int blk = (int)blockIdx.x + pdl_wait();
-    constexpr int kWords = sizeof(DevStatus) / sizeof(int);
     const int t = threadIdx.x + blk;
-    if (t < kWords) reinterpret_cast<volatile int*>(&out->build)[t] = reinterpret_cast<const volatile int*>(st)[t];
-    __threadfence_system();
-    __syncwarp();
-    if (t == 0) *reinterpret_cast<volatile int*>(&out->ready) = 1;
+    if (t < kStatusWords) reinterpret_cast<volatile int*>(&out->build)[t] = reinterpret_cast<const volatile int*>(st)[t];
 }
 
 // A list build's status, read back: the locals outside the grid get empty lists, the two-phase
@@ -1567,7 +1565,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
         else launch_build_list<0>(s, s.ref.b[s.ac], a, la, links);
         launched(K_NLIST);
         prof_end(K_NLIST);
-        *static_cast<volatile int*>(&s.status_host->ready) = -1;
+        for (int k = 0; k < kStatusWords; ++k) reinterpret_cast<volatile int*>(&s.status_host->build)[k] = -1;
         launch(s, 1, 32, 0, k_status_out, s.status_dev, s.status_host);
         launched(K_MISC);
         if (defer && attempt == 0) {
@@ -1588,7 +1586,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
 int resolve_lists(State& s) {
     if (!s.status_pending) return 0;
     s.status_pending = false;
-    if (!await_word(s, &s.status_host->ready)) return -1;  // a latched error
+    if (!await_words(s, &s.status_host->build, kStatusWords)) return -1;  // a latched error
     const bool outside = s.status_host->build.out_local > 0;
     if (finish_build(s, s.status_half) == 0) return outside ? 1 : 0;
     // the capacity was short: the build again, on the grown lists

@@ -102,12 +102,13 @@ struct DevStatus {
     int max_nb;         // longest neighbour list of the last build (zeroed before each build)
 };
 
-// Page-locked words that kernels store straight to and the host polls (await_word): -1 before.
+// Page-locked words that kernels store straight to and the host polls (await_words): -1 until then, so
+// that no store has to be ordered before another.
 struct HostStatus {
-    DevStatus build;  // of the last list build, valid once `ready` is 1
-    int ready;
+    DevStatus build;  // of the last list build
     int nghost;       // ghosts of the border pass in flight
 };
+constexpr int kStatusWords = sizeof(DevStatus) / sizeof(int);
 
 // periodic images a local can push (two-phase: its own first-pass images, one per face
 // it is near; exact: all its images, up to seven where the box is wider than two
@@ -330,7 +331,7 @@ void one_sided_lists(State& s);  // half lists as the reference holds them (no-o
 // completes a deferred list build: 0 when the lists stand, 1 when they were rebuilt (a force
 // kernel launched on them speculatively returned without writing), -1 on an error
 int resolve_lists(State& s);
-bool await_word(State& s, int* word);  // false: still -1 after the stream's work
+bool await_words(State& s, void* words, int n);  // false: one still -1 after the stream's work
 void run_force_lj(State& s, const PendingForce& p, bool fuse_final, double dt);
 void run_force_dem(State& s, const PendingForce& p);
 // kick_dt >= 0: the previous step's final kick of kick_dt is applied first (held back by
