@@ -1240,9 +1240,10 @@ bool grow_atoms(State& s, int need);  // api.cu
 // earlier than after a copy and an event, and the kernels keep following one another without either
 // between them.  When they do not come (a failed launch, a long queue ahead) the stream's work is
 // waited for.  A rebuild of eight kernels with two such waits, by copies and events -> by words stored (us
-// on top of an ordinary step): 256 atoms 54 -> 43, 2,048 55 -> 42, 16,384 65 -> 54, 131,072 143 -> 133,
-// half-filled box of 524,288 433 -> 422, granular gas of 260,800 162 -> 149; at a rebuild every 20 steps
-// 7.24 -> 6.65 us a step at 256 atoms, 14.0 -> 13.6 at 16,384, 44.4 -> 43.75 at 131,072.
+// on top of an ordinary step): 256 atoms 54 -> 40, 2,048 55 -> 40, 16,384 65 -> 51, 131,072 143 -> 130,
+// half-filled box of 524,288 433 -> 421, granular gas of 260,800 162 -> 147; at a rebuild every 20 steps
+// 7.24 -> 6.44 us a step at 256 atoms, 14.0 -> 13.4 at 16,384, 44.4 -> 43.5 at 131,072.  A fence after
+// the stores, with one word for all of them, took 2 us.
 bool await_words(State& s, void* words, int n) {
     const volatile int* const w = static_cast<const volatile int*>(words);
     const auto start = std::chrono::steady_clock::now();
