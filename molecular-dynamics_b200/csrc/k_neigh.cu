@@ -23,6 +23,7 @@
 // which makes list order -- and hence FP64 force summation order -- equal to
 // the reference's.
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cstdio>
@@ -483,6 +484,7 @@ constexpr uint32_t kPadCode = 42u;          // dk = +1 on every axis
 struct NlArgs {
     double cut2;  // cutoff^2 (FP64, the reference's membership test)
     float cut;
+    float wide2;  // an FP32 window that reaches it may hold pairs of |dk| > 1 (far_homes)
     int nbcap, stride, N, ncells, nx, nxy;
     int two;  // half lists: local pairs from both sides (two_sided)
     double alo[3], spacing;
@@ -550,6 +552,43 @@ __device__ __forceinline__ void drain(uint32_t* buf, int& nb, int& out, int i, u
         nb = 0;
         __syncwarp();
     }
+}
+
+// The lists of homes hb .. hb + hn - 1, one of them far outside the cell: the binning tests only the
+// flattened cell index, so a coordinate may be anything, infinite too.  The FP32 margin grows with it,
+// and past wide2 the window takes in pairs of |dk| > 1, whose entries do not give back the candidate's
+// slot.  Every candidate takes the FP64 test here (rare: out of line, so that the walk keeps its registers).
+// both: local candidates below it always pass a half list's reference test (two-sided lists).
+template <int HM>
+__device__ __noinline__ int far_homes(const double4* __restrict__ pos, const int* __restrict__ ref,
+                                      const int* __restrict__ rbk, int* __restrict__ nbn,
+                                      uint32_t* __restrict__ nbl, double cut2, int nbcap, int stride, int both,
+                                      int hb, int hn, int nr, const int* rstart, const int* rpre) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
+    int most = 0;
+    for (int i = hb + (int)(threadIdx.x >> 5); i < hb + hn; i += kNlWarps) {
+        const int rb = __ldg(rbk + i), iref = HM ? __ldg(ref + i) : 0, M = rpre[nr];
+        int cnt = 0, r = 0;
+        for (int m0 = 0; m0 < M; m0 += 32) {
+            const int m = m0 + lane;
+            while (m < M && rpre[r + 1] <= m) ++r;
+            const int slot = m < M ? rstart[r] + m - rpre[r] : i;
+            const bool may = slot != i && (!HM || slot < both || __ldg(ref + slot) < iref);
+            const bool take = may && exact_within(pos, i, slot, cut2);
+            const unsigned hits = __ballot_sync(0xffffffffu, take);
+            const int k = cnt + __popc(hits & lt);
+            if (take && k < nbcap)
+                nbl[nl_index(k, i, stride)] =
+                    ((uint32_t)slot << kCodeBits) + (uint32_t)(rel_code(__ldg(rbk + slot), rb) + kCodeBias);
+            cnt += __popc(hits);
+        }
+        if (lane < ((-cnt) & 3) && cnt + lane < nbcap)  // the last quad's padding
+            nbl[nl_index(cnt + lane, i, stride)] = ((uint32_t)i << kCodeBits) | kPadCode;
+        if (lane == 0) nbn[i] = cnt;
+        most = max(most, cnt);
+    }
+    return most;
 }
 
 template <int HM>
@@ -667,6 +706,11 @@ k_build_list(const double4* __restrict__ pos, const int* __restrict__ ref, const
         }
         __syncthreads();  // ranges and homes are in place
         const int nr = s_nr, M = s_rpre[nr];
+        if (!(s_box[1].w < a.wide2)) {
+            maxcnt = max(maxcnt, far_homes<HM>(pos, ref, rbk, nbn, nbl, a.cut2, a.nbcap, a.stride, a.two ? a.N : 0, hb, hn,
+                                               nr, s_rstart, s_rpre));
+            continue;
+        }
 
         for (int t0 = 0; t0 < M; t0 += kNlTile) {
             // the slots of the tile's candidates, range by range
@@ -1543,6 +1587,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     NlArgs a;
     a.cut2 = cutoff * cutoff;
     a.cut = (float)cutoff;
+    a.wide2 = (float)std::max(g.rb_h * g.rb_h * (1.0 - 1e-6), a.cut2 * (1.0 + 1e-4));
     a.N = s.N;
     a.ncells = g.ncells;
     a.nx = g.nx;
