@@ -1540,7 +1540,7 @@ __global__ void k_status_out(const DevStatus* st, HostStatus* out) {
 // A list build's status, read back: the locals outside the grid get empty lists, the two-phase
 // chain and image-map state of the links; 0 when the lists stand, 1 when the capacity was short
 // (grown: the build is to be redone).
-static int finish_build(State& s, bool half) {
+static int finish_build(State& s) {
     const Geometry& g = s.geo;
     if (s.status_host->build.out_local > 0) {
         int first_out = 0;
@@ -1558,7 +1558,6 @@ static int finish_build(State& s, bool half) {
     s.max_list = mx;
     if (mx <= s.nb_cap) {
         s.lists_valid = 1;
-        s.lists_half = half;
         return 0;
     }
     if (s.lists_two) {  // one-sided lists may still fit
@@ -1598,6 +1597,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
     for (int attempt = 0; attempt < 8; ++attempt) {
         a.nbcap = s.nb_cap;
         a.two = s.lists_two = half && two_sided(s);
+        s.lists_half = half;  // known from the launch on: a deferred build's lists are used before its status is read
         if (attempt > 0 || !s.build_zeroed)  // else zeroed by the binning's reorder kernel
             TMD_CUDA(cudaMemsetAsync(&s.status_dev->max_nb, 0, sizeof(int), s.stream));
         s.build_zeroed = false;
@@ -1623,7 +1623,7 @@ int run_build_lists(State& s, bool half, double cutoff, bool defer) {
             return 0;
         }
         TMD_CUDA(cudaStreamSynchronize(s.stream));
-        if (finish_build(s, half) == 0) return 0;
+        if (finish_build(s) == 0) return 0;
     }
     set_error(2, "neighbour list capacity did not converge");
     return -1;
@@ -1634,7 +1634,7 @@ int resolve_lists(State& s) {
     s.status_pending = false;
     if (!await_words(s, &s.status_host->build, kStatusWords)) return -1;  // a latched error
     const bool outside = s.status_host->build.out_local > 0;
-    if (finish_build(s, s.status_half) == 0) return outside ? 1 : 0;
+    if (finish_build(s) == 0) return outside ? 1 : 0;
     // the capacity was short: the build again, on the grown lists
     return run_build_lists(s, s.status_half, s.lists_cutoff) == 0 ? 1 : -1;
 }
