@@ -728,8 +728,10 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
         const int nquad = (n + 3) >> 2;
         const int rounds = __reduce_max_sync(0xffffffffu, (nquad + L - 1) / L);
         // the next round's gathers are in flight while this one's forces are added, and the quad of the
-        // round after that
-        const uint4 empty = make_uint4(0u, 0u, 0u, 0u);
+        // round after that; past the list's end the atom itself (as its padding), never another atom, whose
+        // non-finite del times f = 0 would reach the sums
+        const uint32_t self = (uint32_t)(act ? i : 0) << kCodeBits;
+        const uint4 empty = make_uint4(self, self, self, self);
         uint4 eq = sub < nquad ? list_quad(nbl, sub, i, a.stride) : empty;
         uint4 en = sub + L < nquad ? list_quad(nbl, sub + L, i, a.stride) : empty;
         float4 rj[kB32];
@@ -788,6 +790,7 @@ k_lj_mixed_lanes(const float4* __restrict__ pos32, const double4* __restrict__ p
             }
             __syncwarp();
         }
+        if (n == 0) acc = 0.f;  // no pairs, whatever the atom's own position
         const int base = lane & ~(L - 1);
         const float fx = __shfl_sync(0xffffffffu, acc, base), fy = __shfl_sync(0xffffffffu, acc, base + 1),
                     fz = __shfl_sync(0xffffffffu, acc, base + 2);
