@@ -1468,14 +1468,22 @@ void flush_links(State& s) {
 // Which list kernel: a block per cell from 8.5 locals per filled cell on.  Measured on LJ liquids of
 // 131,072 atoms with smaller cutoffs, block per cell / eight lanes per home, us: 2.8 per cell 158 / 53,
 // 4.9 112 / 69, 7.8 94 / 87, 11.7 85 / 112, 18.5 91 / 158; the same line at 16,384 and 442,368 atoms.
-// Below 4,096 locals the block per cell is as fast or faster at every density.  The filled cells are
-// those of the last binning whose status was read (the results are the same either way); before the
-// first one the box's mean density stands in.
+// Below 4,096 locals the block per cell is as fast or faster at every density where few cells are empty.
+// An empty cell's block costs 0.52 ns, one that holds few locals 2 ns, so the eight lanes take over where
+// that outweighs their longer chain (up to 9 us, by density) and their cost per home at high density.
+// Gas of 500 locals in 148,877 cells 82 / 8.6 us, of 4,000 in 6,859 21 / 10.7; a liquid cluster of 4,000 in
+// 32,768 25.0 / 21.2, in 148,877 82 / 21, of 32,000 in 32,768 37 / 44, in 59,319 48 / 43, of 108,000 in
+// 97,336 101 / 111, in 148,877 125 / 111.  (A warp per cell, as earlier: 25, 12.7, 49, 57, 59, 62, 110, 111.)
+// The filled cells are those of the last binning whose status was read (the results are the same either
+// way); before the first one the box's mean density stands in, at most a cell per local.
 static bool sparse_cells(const State& s) {
     const Geometry& g = s.geo;
-    if (s.N <= 4096) return false;
-    if (s.cells_filled > 0) return (double)s.N < 8.5 * s.cells_filled;
-    return (double)s.N * g.spacing * g.spacing * g.spacing < 8.5 * g.len[0] * g.len[1] * g.len[2];
+    const double box = g.len[0] * g.len[1] * g.len[2] / (g.spacing * g.spacing * g.spacing);
+    const double filled = s.cells_filled > 0 ? s.cells_filled : std::min((double)s.N, box);
+    const double each = s.N / filled, over = each - 8.5;
+    if (s.N > 4096 && over < 0.0) return true;
+    const double saved = 0.52 * (g.ncells - filled) + (over < 0.0 ? 1.5 * filled : 0.0);  // ns
+    return saved > 2000.0 + 500.0 * each + 0.05 * s.N * std::max(over, 0.0);
 }
 
 template <int HM>
