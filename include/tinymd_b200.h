@@ -86,7 +86,8 @@ void md_distribute_particles(void);
  * is read while it runs, the build and force redone on an overflow; a warning of the build is
  * latched by then, or by the next call that reads state or the error code. */
 void md_assemble_neighborlists(bool half_neighborlist, double cutoff_distance);
-/* anydsl_includes.h:22, core/runtime.impala:97-102 */
+/* anydsl_includes.h:22, core/runtime.impala:97-102.  Up to 64 device blocks and 1 GiB stay with the library
+ * for the next grid; md_release_device_memory or md_mpi_finalize gives them back to the device. */
 void md_deallocate_grid(void);
 /* anydsl_includes.h:23-24, core/runtime.impala:146-156 */
 void md_print_grid(void);
@@ -107,7 +108,8 @@ void md_compute_dem(bool half_neighborlist, double cutoff_distance, double dampi
  * (TINYMD_DEVICE, else the launcher's local rank) and picks the transport of the halo data:
  * NCCL when every rank has its own GPU, else page-locked host buffers over the TCP mesh
  * (TINYMD_COMM=auto|socket|nccl).  Without those variables the run has one rank.
- * md_mpi_finalize releases the grid and the connections.  Several ranks run full neighbour
+ * md_mpi_finalize releases the grid, the device blocks kept from earlier grids and the connections.
+ * Several ranks run full neighbour
  * lists and exact ghosts; md_report_* print sums (times: maxima) over the ranks on rank 0. */
 void md_mpi_initialize(void);
 void md_mpi_finalize(void);
@@ -217,6 +219,10 @@ void md_profile_reset(void);
 long long md_kernel_launches(void);
 /* Device bytes asked for by the current grid (blocks kept from earlier grids are not counted). */
 long long md_device_bytes(void);
+/* Gives the device blocks that closed grids left with the library back to the device, for a program
+ * that needs the room for something else (an allocation of the library's own that fails does this by
+ * itself; one of another library cannot).  The current grid, if there is one, is not touched. */
+void md_release_device_memory(void);
 
 /* Runs `steps` timesteps of the md driver loop (main.cpp:715-776) natively:
  * initial integration, ghost refresh -- or, when (step0 + k + 1) is a

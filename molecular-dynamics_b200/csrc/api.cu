@@ -1532,6 +1532,7 @@ int md_profile_get(int id, long long* launches, double* total_ms) {
 void md_profile_reset(void) { prof_reset(); }
 long long md_kernel_launches(void) { return g_state.launches; }
 long long md_device_bytes(void) { return g_state.dev_bytes; }
+void md_release_device_memory(void) { release_kept_blocks(); }
 
 int md_get_neighbor_lists(int* sizes, int* lists, int capacity) {
     State& s = g_state;

@@ -83,6 +83,7 @@ _EXTENSION_API = {
     "md_profile_reset": (None, []),
     "md_kernel_launches": (_c_ll, []),
     "md_device_bytes": (_c_ll, []),
+    "md_release_device_memory": (None, []),
     "md_get_neighbor_lists": (_c_int, [_vp, _vp, _c_int]),
     "md_get_ghost_info": (_c_int, [_vp, _vp, _vp, _vp]),
     "md_get_state": (_c_int, [_vp, _vp, _vp]),
@@ -309,7 +310,14 @@ class Simulation:
         return m, x, v, f
 
     def close(self):
+        """Frees the grid; up to 1 GiB of its device blocks stay for the next one (release_device_memory)."""
         self.lib.md_deallocate_grid()
+
+
+def release_device_memory(lib=None):
+    """Gives the device memory that closed grids left with the library back to the device, so that other
+    allocators of the process (torch) can have it.  An open grid is not touched."""
+    (lib or load()).md_release_device_memory()
 
 
 def is_oracle(lib):
