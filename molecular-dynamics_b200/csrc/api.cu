@@ -826,6 +826,7 @@ int md_initialize_grid(double const* masses, Vector3D const* positions, Vector3D
     s.pc = s.vc = s.ac = 0;
     s.lists_valid = 0;
     s.lists_two = s.two_short = false;
+    s.force_seen = false;
     s.cells_filled = 0;
     s.pend_init = false;
     s.pend_force = PendingForce();
@@ -1077,6 +1078,7 @@ void md_compute_lennard_jones(bool half, double rc, double eps, double sigma) {
     p.sigma = sigma;
     s.pend_force = p;
     s.force_cfg = p;
+    s.force_seen = true;
     s.last_rc = rc;
     s.last_eps = eps;
     s.last_sigma = sigma;
@@ -1098,6 +1100,7 @@ void md_compute_dem(bool half, double rc, double damping_n, double damping_t, do
     p.mu = friction;
     s.pend_force = p;
     s.force_cfg = p;
+    s.force_seen = true;
 }
 
 void md_final_integration(double dt) {

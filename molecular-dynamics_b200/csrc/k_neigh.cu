@@ -1506,9 +1506,11 @@ void launch_build_list(State& s, const int* ref, const NlArgs& a, const LinkArgs
 // kept, rebuild every 20 steps included): 256 atoms 26.8 -> 10.8, 2,048 27.3 -> 11.7, 16,384 28.2 -> 18.9,
 // 48,668 44.3 -> 37.9, 131,072 83.1 -> 57.4, 442,368 240 -> 158, 864,000 447 -> 274.  The list build
 // stays within 2 %.  Not for the other half kernels (DEM's lists are short, the mixed form adds four
-// floats at once), nor where the longer lists outgrow the capacity of the reference's.
+// floats at once), nor where the longer lists outgrow the capacity of the reference's.  The force is this
+// grid's last one; the lists built before its first are DEM's when the contact model is set.
 static bool two_sided(const State& s) {
-    return s.precision == 0 && !(s.force_cfg.valid && s.force_cfg.dem) && !s.two_short;
+    const bool dem = s.force_seen ? s.force_cfg.dem : s.dem_fixed != 0;
+    return s.precision == 0 && !dem && !s.two_short;
 }
 
 // Drops the entries that the reference's half lists do not hold, in place and in order: a local

@@ -268,6 +268,7 @@ struct State {
 
     PendingForce pend_force;
     PendingForce force_cfg;   // parameters of the last md_compute_* call
+    bool force_seen = false;  // force_cfg is of this grid, not of an earlier one
     bool pend_init = false;
     double pend_dt = 0.0;
     // a full-list LJ force whose final integration was requested: launched when the next
