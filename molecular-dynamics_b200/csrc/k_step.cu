@@ -1604,13 +1604,14 @@ StepArgs step_args(const State& s, double dt) {
 // steps included), 1 / 4 / 8 / 16 lanes:
 //   mixed  256 atoms 15.6 /  9.2 /  8.3 /  8.0    2,048 16.6 / 10.3 /  8.9 /  9.0    5,148 18.0 / 10.9 / 10.4 / 11.3
 //         10,976     17.9 / 12.8 / 13.1 / 18.3   16,384 17.7 / 14.0 / 15.7 / 21.5   29,716 20.0 / 19.4 / 25.6
-//         55,296     22.7 / 32.9 (2 lanes: 29,716 19.2, 55,296 25.7)
+//         55,296     22.7 / 32.9 (2 lanes: 29,716 19.2, 55,296 25.7); later, around the line, 1 / 4 lanes:
+//         28,880     18.9 / 18.3   29,716 19.9 / 18.6   30,400 18.8 / 18.5   32,000 18.6 / 18.8   33,600 18.8 / 19.8
 //   FP64   256 atoms 19.2 /  9.6 /  7.4 /  6.8    2,048 21.4 / 10.2 /  7.8 /  7.8    5,148 22.3 / 10.8 /  9.8 / 10.7
 //         10,976     22.4 / 12.3 / 13.1 / 18.0   29,716 24.2 / 20.7 / 27.6           42,592 25.2 / 30.7
 int force_lanes(int N, bool mixed) {
     if (N <= (mixed ? 1024 : 2048)) return 16;
     if (N <= 8192) return 8;
-    return N <= (mixed ? 29000 : 36000) ? 4 : 1;
+    return N <= (mixed ? 31000 : 36000) ? 4 : 1;
 }
 
 // Thread-per-atom kernels with the next quad's gathers in flight.  FP64: 30 % less time per wave of

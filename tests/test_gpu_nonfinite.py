@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("axis,value", [(0, np.nan), (slice(3), np.nan), (1, -np.inf), (2, -np.inf)])
-@pytest.mark.parametrize("cells", [(6, 5, 6), (13, 12, 13), (19, 19, 20), (20, 19, 20)])
+@pytest.mark.parametrize("cells", [(6, 5, 6), (13, 12, 13), (19, 19, 20), (21, 19, 21)])
 def test_mixed_forces_beside_a_nonfinite_local(product, cuda_device, cells, axis, value):
     m, x, v, world, rank = tinymd.setup_particles("default", cells, lib=product)
     lo, length = world[0::2], world[1::2] - world[0::2]
