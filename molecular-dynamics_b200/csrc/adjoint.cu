@@ -391,7 +391,8 @@ void finish_move(State& s, int t, bool pushed) {
 // The velocity-Verlet steps t0 .. t1-1 from x_t0 (with its force) on: one kernel per step, the force at
 // x_{t+1}, its kick and the integration to x_{t+2}, as the driver's loop runs it; after_step(t) is called
 // with x_{t+1}, v_{t+1} in place wherever stop(t) asks for it, and after the last step.  move(t) is
-// called before the launch that writes x_{t+1}.
+// called before the launch that writes x_{t+1}.  With the contact model set the force and the integration
+// run apart: only run_integrate refreshes the ghosts' velocities, which that model's grid holds.
 template <class Stop, class After, class Move>
 void run_steps(State& s, int t0, int t1, bool last_force, Stop stop, After after_step, Move move) {
     bool moved = false;  // x_{t+1} is there already
@@ -402,7 +403,7 @@ void run_steps(State& s, int t0, int t1, bool last_force, Stop stop, After after
             run_integrate(s, cfg.dt, !ren);
             finish_move(s, t, true);
         }
-        moved = t + 1 < t1 && !stop(t);
+        moved = t + 1 < t1 && !stop(t) && s.dem_fixed == 0;
         if (moved) {
             move(t + 1);
             run_force_lj_init(s, force_params(), cfg.dt, cfg.dt);
