@@ -6,7 +6,7 @@
 //   * neighbour-list build (core/neighborlist.impala:1-78): a block per cell,
 //     the stencil's candidates filtered by the homes' bounding box and staged
 //     in shared memory, a warp testing 32 of them against a home at once; or
-//     eight lanes per home where cells hold few atoms
+//     eight lanes per home where cells hold few atoms or most hold none
 //
 // Ghost order.  The reference runs six passes (x+, x-, y+, y-, z+, z-); a
 // pass scans locals then all earlier ghosts in order and appends the ones
